@@ -8,19 +8,19 @@
 // interpolation of its four neighbours (floor / ceil corners).  The ray sum is
 // scaled by step_size * dx.
 //
-// FP32 path (see fp_cast_f32 for the warp layout).  The sample range of each axis is decided
-// exactly as the reference decides it: in 32.32 fixed point where that is
+// FP32 path (fp_cast_rows_f32 for steps up to half a pixel, fp_cast_f32 above and
+// where the copies do not fit).  The sample range of each axis is decided exactly as the reference decides it: in 32.32 fixed point where that is
 // certain, and by the reference's own FP64 accumulation (acc_advance, jumping
 // binade to binade) for the few samples within a hair of an image edge
 // (fp_setup.cuh).  The running position is monotone in k, so each axis keeps a
-// contiguous range and the ray keeps their intersection.  Inside it the thread
-// marches both coordinates in fixed point (two 64-bit adds a sample) and
-// interpolates in FP32; positions differ from the reference's FP64 ones by
+// contiguous range and the ray keeps their intersection.  Inside it both
+// coordinates are fixed point and the interpolation FP32; positions differ from the reference's FP64 ones by
 // ~1e-9 pixel, which moves the interpolation weights by as much (continuous at
 // pixel boundaries).
 //
 // FP64 path: one thread per ray, the reference's loop (FP64 positions and
 // inclusion test, FP64 interpolation and sum).
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -101,6 +101,160 @@ __global__ void __launch_bounds__(kCastThreads)
     }
 }
 
+// ---- FP32, small steps: one closed form per image row ------------------------
+// A ray marched along its steeper axis takes 1 / (|sin| or |cos| * step_size)
+// samples between two image rows, and crosses at most one column boundary on
+// the way.  The bilinear interpolant is (1 - v) P_j(x) + v P_j+1(x) there, each
+// P piecewise linear with its one knot at that boundary, and the samples are
+// arithmetic progressions in x and v, so their sum is six pixels with weights
+// that the sums of 1, k and k^2 over the samples before and after the knot
+// give: the work is per row crossed (9.3 samples a row on average at a step of
+// 0.125 pixel) instead of per sample.  A sample put on the wrong side of a row
+// or of the knot lies within FP32 rounding of it, where both forms agree.
+//
+// One lane per ray, a block's lanes on adjacent channels of one view, so a
+// warp's pixels of a row are adjacent; rays marched in x read the transposed
+// copy.  Both copies have a border of kCastPad zeros around the image (the
+// fixed-point positions may sit a hair outside it, where the weight is ~0), so
+// the loop has no clamps.  Issue bound: ~75 instructions per ray and row, 67 %
+// of the issue slots (512^2 x 720 x 729 at a step of 0.125: 2450 -> 468 us).
+// Blocks of 64 rays: 128 took as long, 32 were 2 % slower; fewer registers for
+// more warps spilled (20 blocks of 64 a SM: 526 us).
+constexpr int kCastPad = 2;
+constexpr int kRowThreads = 64, kRowBlocks = 16;  // rays a block, blocks an SM
+
+// The padded image and its padded transpose, 32 x 32 tiles of padded pixels.
+__global__ void __launch_bounds__(256)
+    cast_pad(const float* __restrict__ img, float* __restrict__ rows, float* __restrict__ cols, int nx, int ny)
+{
+    __shared__ float t[32][33];
+    const int wx = nx + 2 * kCastPad, wy = ny + 2 * kCastPad;
+    const size_t off = static_cast<size_t>(blockIdx.z) * nx * ny, poff = static_cast<size_t>(blockIdx.z) * wx * wy;
+    const int x0 = blockIdx.x * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    // grid.y strides over the rows of tiles
+    for (int y0 = blockIdx.y * 32; y0 < wy; y0 += gridDim.y * 32) {
+        for (int r = ty; r < 32; r += 8) {
+            const int x = x0 + tx - kCastPad, y = y0 + r - kCastPad;
+            const float v = x >= 0 && x < nx && y >= 0 && y < ny ? img[off + static_cast<size_t>(y) * nx + x] : 0.0f;
+            t[r][tx] = v;
+            if (x0 + tx < wx && y0 + r < wy) rows[poff + static_cast<size_t>(y0 + r) * wx + x0 + tx] = v;
+        }
+        __syncthreads();
+        for (int r = ty; r < 32; r += 8)
+            if (x0 + r < wx && y0 + tx < wy) cols[poff + static_cast<size_t>(x0 + r) * wy + y0 + tx] = t[tx][r];
+        __syncthreads();
+    }
+}
+
+// The bits of 1 + the fraction of a 32.32 fixed-point value (its top 23 bits).
+__device__ __forceinline__ float cast_one_frac(unsigned long long X)
+{
+    return __uint_as_float(0x3F800000u | (static_cast<unsigned>(X) >> 9));
+}
+
+// One lane's ray of the row-by-row march: its first sample and step on the
+// marched axis (M, MS) and across it (C, CS; mirrored where the ray runs down
+// the image, so that CS >= 0), both 32.32 fixed point, and its samples.
+struct CastRay {
+    unsigned long long M, C;
+    unsigned MS, CS;  // below 1 pixel
+    int left;
+};
+
+// The sum over a ray's samples; the warp's lanes take the image rows together
+// (a lane waits for the row its ray starts on), so that each load reads
+// adjacent pixels of one row.  P: the copy, at pixel (0, 0); w: its row stride;
+// Dir: the direction of C in the image.
+template <int Dir>
+__device__ __forceinline__ float cast_march(CastRay r, const float* __restrict__ P, int w)
+{
+    const float a = static_cast<float>(r.CS) * 2.3283064365386963e-10f;  // 2^-32
+    const float b = static_cast<float>(r.MS) * 2.3283064365386963e-10f;
+    const float inv_a = __fdividef(1.0f, a), inv_b = __fdividef(1.0f, b);
+    const float nab3 = a * b * (-1.0f / 3.0f);
+    const float2 a2 = make_float2(a, a), nab2 = make_float2(nab3, nab3);
+    const float2 half2 = make_float2(0.5f, 0.5f), mhalf2 = make_float2(-0.5f, -0.5f);
+    const float2 two2 = make_float2(2.0f, 2.0f), minus1 = make_float2(-1.0f, -1.0f);
+    float2 sum = make_float2(0.0f, 0.0f);
+    int j = __reduce_min_sync(0xffffffffu, r.left > 0 ? static_cast<int>(r.M >> 32) : 0x7fffffff);
+    for (; __any_sync(0xffffffffu, r.left > 0); ++j) {
+        const int row = static_cast<int>(r.M >> 32), col = static_cast<int>(r.C >> 32);
+        if (r.left <= 0 || row > j) continue;
+        const float* p = P + (Dir > 0 ? row * w + col : row * w - col);
+        const float* p1 = p + w;
+        const float v1 = cast_one_frac(r.M), u1 = cast_one_frac(r.C);
+        const float d0 = 2.0f - u1, v0 = v1 - 1.0f;  // distance to the knot, position past the row
+        // samples in this row, and those of them before the knot
+        const int m = min(r.left, __float2int_ru((2.0f - v1) * inv_b));  // >= 1: v1 < 2
+        const int q = min(m, __float2int_ru(d0 * inv_a));
+        const float2 B = make_float2(__ldg(p), __ldg(p1));
+        const float2 K = make_float2(__ldg(p + Dir), __ldg(p1 + Dir));
+        float2 A = make_float2(0.0f, 0.0f);  // past the knot: only where a sample is
+        if (q < m) A = make_float2(__ldg(p + 2 * Dir), __ldg(p1 + 2 * Dir));
+        // over the first q and over all m samples, packed: x, the sum of the
+        // positions past the knot -d0 + k a, and y, minus the sum of v times it
+        // (v = v0 + k b)
+        const float2 n = make_float2(static_cast<float>(q), static_cast<float>(m));
+        const float2 s1 = __fmul2_rn(n, __ffma2_rn(n, half2, mhalf2));
+        const float2 s3 = __fmul2_rn(s1, __ffma2_rn(n, two2, minus1));
+        const float vd = v0 * d0, cr = fmaf(d0, b, -v0 * a);
+        const float2 x = __ffma2_rn(a2, s1, __fmul2_rn(n, make_float2(-d0, -d0)));
+        const float2 y = __ffma2_rn(nab2, s3, __ffma2_rn(make_float2(cr, cr), s1, __fmul2_rn(n, make_float2(vd, vd))));
+        const float sv = fmaf(b, s1.y, n.y * v0);  // sum of v
+        // weights of the pixel before the knot, after it and at it, rows j and j + 1
+        const float2 wb = make_float2(-y.x - x.x, y.x);
+        const float wa1 = y.x - y.y;
+        const float2 wa = make_float2((x.y - x.x) - wa1, wa1);
+        const float2 wk = make_float2((n.y - sv) - wb.x - wa.x, sv - wb.y - wa.y);
+        sum = __ffma2_rn(wb, B, sum);
+        sum = __ffma2_rn(wa, A, sum);
+        sum = __ffma2_rn(wk, K, sum);
+        r.left -= m;
+        r.M += static_cast<unsigned long long>(static_cast<unsigned>(m)) * r.MS;
+        r.C += static_cast<unsigned long long>(static_cast<unsigned>(m)) * r.CS;
+    }
+    return sum.x + sum.y;
+}
+
+__global__ void __launch_bounds__(kRowThreads, kRowBlocks)
+    fp_cast_rows_f32(const float* __restrict__ rows, const float* __restrict__ cols, float* __restrict__ proj,
+                     const double* __restrict__ sincos, const double* __restrict__ begins,
+                     const int* __restrict__ nsteps, int ns, int nx, int ny, unsigned chunks, double step_size,
+                     float scale, size_t proj_stride)
+{
+    const unsigned ia = blockIdx.x / chunks;
+    const int is = static_cast<int>((blockIdx.x - ia * chunks) * kRowThreads + threadIdx.x);
+    const size_t ray = static_cast<size_t>(ia) * ns + is;
+    const double sx = step_size * sincos[2 * ia], sy = step_size * sincos[2 * ia + 1];
+    // a view's rays are marched along one axis, turned so that M runs up
+    const bool along_y = fabs(sy) >= fabs(sx);
+    const bool turn = (along_y ? sy : sx) < 0.0, down = ((along_y ? sx : sy) < 0.0) != turn;
+    CastRay r{0, 0, 0, 0, 0};
+    if (is < ns) {
+        const int nstep = nsteps[ray];
+        if (nstep > 0) {
+            int kx0, kx1, ky0, ky1;
+            long long X, SX, Y, SY;
+            axis_range(begins[2 * ray], sx, nstep, nx, &X, &SX, &kx0, &kx1);
+            axis_range(begins[2 * ray + 1], sy, nstep, ny, &Y, &SY, &ky0, &ky1);
+            const int k0 = max(kx0, ky0), k1 = min(kx1, ky1), ks = turn ? k1 : k0;
+            r.left = max(0, k1 - k0 + 1);
+            const long long ms = along_y ? SY : SX, cs = along_y ? SX : SY;
+            const long long c = (along_y ? X : Y) + ks * cs;
+            r.M = (along_y ? Y : X) + ks * ms;
+            r.MS = static_cast<unsigned>(turn ? -ms : ms);
+            r.C = down ? -c : c;
+            r.CS = static_cast<unsigned>(down != turn ? -cs : cs);
+        }
+    }
+    const int w = (along_y ? nx : ny) + 2 * kCastPad;
+    const float* P = (along_y ? rows : cols) +
+                     static_cast<size_t>(blockIdx.y) * (nx + 2 * kCastPad) * (ny + 2 * kCastPad) +
+                     static_cast<size_t>(kCastPad) * w + kCastPad;
+    const float sum = down ? cast_march<-1>(r, P, w) : cast_march<1>(r, P, w);
+    if (is < ns) proj[blockIdx.y * proj_stride + ray] = sum * scale;
+}
+
 __global__ void __launch_bounds__(kCastThreads)
     fp_cast_f64(const double* __restrict__ img, double* __restrict__ proj, const double* __restrict__ sincos,
                 const double* __restrict__ begins, const int* __restrict__ nsteps, int ns, int na, int nx,
@@ -148,6 +302,41 @@ int check_cast(const ctr_par_param* p, double step_size, const void* a, const vo
     return CTR_OK;
 }
 
+// Steps up to this many pixels go row by row (fp_cast_rows_f32): the time does
+// not depend on the step there, that of the sample-by-sample kernel does.  Per
+// call (copies included), row by row against sample by sample:
+//   512^2 x 720 x 729   step 0.125: 468 / 2450 us, 0.5: 466 / 1176, 0.75: 465 / 1040
+//   128^2 x 180 x 190   step 0.125: 51 / 135 us,   0.5: 41 / 57,    0.75: 40 / 45
+//   64^2 x 90 x 96      step 0.125: 34 / 70 us,    0.5: 30 / 33,    0.75: 31 / 28
+constexpr double kCastRowStep = 0.5;
+constexpr int kCastNotRows = -1;
+
+// The row-by-row path of an FP32 call, kCastNotRows where it does not take it.
+int cast_rows(const ctr_par_param* p, double step_size, const float* img, float* proj, const double* sc,
+              const double* begins, const int* nsteps, float scale, int batch, cudaStream_t stream)
+{
+    const size_t wx = static_cast<size_t>(p->nx) + 2 * kCastPad, wy = static_cast<size_t>(p->ny) + 2 * kCastPad;
+    const unsigned chunks = div_up(p->ns, kRowThreads);
+    const size_t blocks = static_cast<size_t>(chunks) * p->na;
+    // the march indexes a copy with 32-bit integers
+    if (step_size > kCastRowStep || wx * wy > 0x7fffffffu || blocks > 0x7fffffffu) return kCastNotRows;
+    float* rows = nullptr;
+    const size_t item = wx * wy;
+    if (cudaMallocAsync(reinterpret_cast<void**>(&rows), 2 * sizeof(float) * item * batch, stream) != cudaSuccess) {
+        cudaGetLastError();  // no room for the copies: sample by sample
+        return kCastNotRows;
+    }
+    float* cols = rows + item * batch;
+    cast_pad<<<dim3(div_up(wx, 32), std::min<size_t>(div_up(wy, 32), 32768), batch), 256, 0, stream>>>(
+        img, rows, cols, static_cast<int>(p->nx), static_cast<int>(p->ny));
+    fp_cast_rows_f32<<<dim3(static_cast<unsigned>(blocks), batch), kRowThreads, 0, stream>>>(
+        rows, cols, proj, sc, begins, nsteps, p->ns, p->nx, p->ny, chunks, step_size, scale,
+        static_cast<size_t>(p->na) * p->ns);
+    const int st = check_launch("fp_par_2d ray casting");
+    cudaFreeAsync(rows, stream);  // after the kernel that reads it
+    return st;
+}
+
 template <typename T>
 int cast_forward(const ctr_par_param* p, double step_size, const T* img, T* proj, const double* sc,
                  const double* begins, const int* nsteps, int batch, cudaStream_t stream)
@@ -157,10 +346,13 @@ int cast_forward(const ctr_par_param* p, double step_size, const T* img, T* proj
     const long long rays = static_cast<long long>(p->na) * p->ns;
     const dim3 grid(static_cast<unsigned>(div_up(static_cast<unsigned long long>(rays), kCastThreads)), batch);
     const size_t is = static_cast<size_t>(p->nx) * p->ny, ps = static_cast<size_t>(p->na) * p->ns;
-    if constexpr (sizeof(T) == 4)
+    if constexpr (sizeof(T) == 4) {
+        const float scale = static_cast<float>(step_size * p->dx);
+        const int rc = cast_rows(p, step_size, img, proj, sc, begins, nsteps, scale, batch, stream);
+        if (rc != kCastNotRows) return rc;
         fp_cast_f32<<<grid, kCastThreads, 0, stream>>>(img, proj, sc, begins, nsteps, p->ns, p->na, p->nx, p->ny,
-                                                       step_size, static_cast<float>(step_size * p->dx), is, ps);
-    else
+                                                       step_size, scale, is, ps);
+    } else
         fp_cast_f64<<<grid, kCastThreads, 0, stream>>>(img, proj, sc, begins, nsteps, p->ns, p->na, p->nx, p->ny,
                                                        step_size, p->dx, is, ps);
     return check_launch("fp_par_2d ray casting");
