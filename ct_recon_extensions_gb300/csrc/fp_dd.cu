@@ -20,7 +20,8 @@
 // length * proj / 2 over channels ceil(left - 0.5) .. floor(right + 0.5); a
 // negative first channel skips the view (the same unsigned index), and
 // channels past ns read on into the next view's row as the reference's
-// unchecked index does (0 past the last view).  One thread per pixel.
+// unchecked index does (0 past the last view).
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 #include <vector>
@@ -40,18 +41,25 @@ __device__ __forceinline__ float dd_frac(long long X)
     return __uint_as_float(0x3F800000u | (static_cast<unsigned>(X) >> 9)) - 1.0f;
 }
 
-// imgT[b][x][y] = img[b][y][x] (32 x 32 tiles)
-__global__ void __launch_bounds__(256) dd_transpose(const float* __restrict__ img, float* __restrict__ imgT, int n)
+// Copies of the image with its lines as rows (rows: image rows, cols: image
+// columns), each row padded with kDdPad zeros; 32 x 32 tiles.
+constexpr int kDdPad = 3;
+__global__ void __launch_bounds__(256)
+    dd_copies(const float* __restrict__ img, float* __restrict__ rows, float* __restrict__ cols, int n)
 {
     __shared__ float t[32][33];
-    const size_t off = static_cast<size_t>(blockIdx.z) * n * n;
+    const size_t off = static_cast<size_t>(blockIdx.z) * n * n, w = n + kDdPad, poff = blockIdx.z * n * w;
     const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int r = ty; r < 32; r += 8)
-        if (x0 + tx < n && y0 + r < n) t[r][tx] = img[off + static_cast<size_t>(y0 + r) * n + x0 + tx];
+    for (int r = ty; r < 32; r += 8) {
+        const int x = x0 + tx, y = y0 + r;
+        const float v = x < n && y < n ? img[off + static_cast<size_t>(y) * n + x] : 0.0f;
+        t[r][tx] = v;
+        if (x < w && y < n) rows[poff + y * w + x] = v;
+    }
     __syncthreads();
     for (int r = ty; r < 32; r += 8)
-        if (y0 + tx < n && x0 + r < n) imgT[off + static_cast<size_t>(x0 + r) * n + y0 + tx] = t[tx][r];
+        if (x0 + r < n && y0 + tx < w) cols[poff + (x0 + r) * w + y0 + tx] = t[tx][r];
 }
 
 // One ray of the forward with the reference's own arithmetic: FP64 edges,
@@ -125,84 +133,175 @@ __global__ void __launch_bounds__(kDdThreads)
 // n-1 dropped after an exact check).  Inside it both edges march in 32.32
 // fixed point, and the covered lengths are FP32 relative to the first
 // interval; everything else varies continuously with the edges.  Lines of
-// column-marching views read the transposed copy, so a warp's loads stay
-// within a few rows.  Rays outside the fixed-point range take dd_ray_exact.
-__global__ void __launch_bounds__(kDdThreads)
-    fp_dd_f32(const float* __restrict__ img, const float* __restrict__ imgT, float* __restrict__ proj,
-              const double* __restrict__ sincos, const double* __restrict__ bo, const int* __restrict__ usex,
-              int ns, int na, int n, double dx, double dy, size_t img_stride, size_t proj_stride)
+// column-marching views read the transposed copy.  Rays outside the
+// fixed-point range take dd_ray_exact.
+//
+// A footprint's width is the same on every line, and up to two pixels (every
+// view when ds <= sqrt(2) dx) it covers at most three intervals: all lines but
+// those at the image's edges run a loop without an interval count or a
+// division, the common width divided out at the end.  One lane per ray, a
+// block's lanes on adjacent channels of one view, the warp's rays on the same
+// line, so that each load reads adjacent pixels.  Issue bound.
+constexpr int kDdRayThreads = 64, kDdUnroll = 4;
+
+// A counted line's tsum / lsum, with the edges' clamps.
+__device__ __forceinline__ float dd_line(const float* __restrict__ line, long long xl, long long xr, int n)
 {
-    const long long ray = static_cast<long long>(blockIdx.x) * kDdThreads + threadIdx.x;
-    if (ray >= static_cast<long long>(na) * ns) return;
-    const int ia = static_cast<int>(ray / ns);
+    const int h = static_cast<int>(xl >> 32);
+    const int i0 = min(max(h, 0), n - 2);
+    // the start relative to interval i0 (clamped: the fixed-point start may
+    // sit a hair outside [0, n-1) where the exact one is inside)
+    const float lr = h == i0 ? dd_frac(xl) : (h < 0 ? 0.0f : 1.0f);
+    const int hr = static_cast<int>(xr >> 32);
+    const float rr = static_cast<float>(hr - i0) + dd_frac(xr);
+    const int ie = min(hr + (static_cast<unsigned>(xr) != 0u ? 1 : 0), n - 1);
+    float tsum = 0.0f, lsum = 0.0f;
+    for (int i = i0; i < ie; ++i) {
+        const float j = static_cast<float>(i - i0);
+        const float len = fmaxf(fminf(j + 1.0f, rr) - fmaxf(j, lr), 0.0f);
+        tsum = fmaf(len, (__ldg(line + i) + __ldg(line + i + 1)) * 0.5f, tsum);
+        lsum += len;
+    }
+    // a counted line always covers part of interval i0; where the clamped
+    // fixed-point edges leave no length, that sliver's trapezoid is the mean
+    return lsum > 0.0f ? tsum / lsum : (__ldg(line + i0) + __ldg(line + i0 + 1)) * 0.5f;
+}
+
+__global__ void __launch_bounds__(kDdRayThreads, 14)
+    fp_dd_f32(const float* __restrict__ img, const float* __restrict__ rows, const float* __restrict__ cols,
+              float* __restrict__ proj,
+              const double* __restrict__ sincos, const double* __restrict__ bo, const int* __restrict__ usex,
+              int ns, unsigned chunks, int n, double dx, double dy, size_t img_stride, size_t proj_stride)
+{
+    const unsigned ia = blockIdx.x / chunks;
+    const int is = static_cast<int>((blockIdx.x - ia * chunks) * kDdRayThreads + threadIdx.x);
+    const size_t ray = static_cast<size_t>(ia) * ns + is;
     const int ux = usex[ia];
-    const float w = static_cast<float>(ux ? fabs(dy / sincos[2 * ia + 1]) : fabs(dx / sincos[2 * ia]));
-    const double* b = bo + 3 * ray;
-    float* out = proj + blockIdx.y * proj_stride + ray;
-    const double off = b[1];
-    double left0 = __dsub_rn(b[0], b[2]), right0 = __dadd_rn(b[0], b[2]);
-    if (left0 > right0) {
-        const double t = left0;
-        left0 = right0;
-        right0 = t;
-    }
-    const int er = static_cast<int>((double_bits(right0) >> 52) & 0x7FF);
-    const int el = static_cast<int>((double_bits(left0) >> 52) & 0x7FF);
-    const int eo = static_cast<int>((double_bits(off) >> 52) & 0x7FF);
-    if (er >= 1043 || el >= 1043 || eo >= 1025 || n < 2) {  // beyond the fixed-point range
-        *out = dd_ray_exact<float>(img + blockIdx.y * img_stride, b, ux, n, n, n) * w;
-        return;
-    }
-    long long XL, S;
-    int k0, k1;
-    axis_range(left0, off, n, n, &XL, &S, &k0, &k1);
-    // a start exactly at n-1 leaves no interval: the range's end there drops
-    if (k0 <= k1) {
-        const double lim = static_cast<double>(n - 1);
-        const long long L = static_cast<long long>(n - 1) << 32, T = tie_units(n);
-        if (off == 0.0) {
-            if (left0 == lim) k1 = k0 - 1;
+    const size_t w = n + kDdPad;
+    const float* I = (ux ? rows : cols) + blockIdx.y * n * w;  // lines are rows of I
+    long long xl = 0, xr = 0, S = 0;
+    int k0 = 1, k1 = 0;  // the lines left to the loop
+    float sum = 0.0f;
+    if (is < ns) {
+        const double* b = bo + 3 * ray;
+        const double off = b[1];
+        double left0 = __dsub_rn(b[0], b[2]), right0 = __dadd_rn(b[0], b[2]);
+        if (left0 > right0) {
+            const double t = left0;
+            left0 = right0;
+            right0 = t;
+        }
+        const int er = static_cast<int>((double_bits(right0) >> 52) & 0x7FF);
+        const int el = static_cast<int>((double_bits(left0) >> 52) & 0x7FF);
+        const int eo = static_cast<int>((double_bits(off) >> 52) & 0x7FF);
+        if (er >= 1043 || el >= 1043 || eo >= 1025 || n < 2) {  // beyond the fixed-point range
+            sum = dd_ray_exact<float>(img + blockIdx.y * img_stride, b, ux, n, n, n);
         } else {
-            const int ke = off > 0.0 ? k1 : k0;
-            const long long X = XL + static_cast<long long>(ke) * S;
-            if (X > L - T && X < L + T) {
-                AccWalk wk{left0, 0};
-                acc_advance(&wk, off, ke);
-                if (wk.x == lim) {
-                    if (off > 0.0) --k1;
-                    else ++k0;
+            long long XL;
+            axis_range(left0, off, n, n, &XL, &S, &k0, &k1);
+            // a start exactly at n-1 leaves no interval: the range's end there drops
+            if (k0 <= k1) {
+                const double lim = static_cast<double>(n - 1);
+                const long long L = static_cast<long long>(n - 1) << 32, T = tie_units(n);
+                if (off == 0.0) {
+                    if (left0 == lim) k1 = k0 - 1;
+                } else {
+                    const int ke = off > 0.0 ? k1 : k0;
+                    const long long X = XL + static_cast<long long>(ke) * S;
+                    if (X > L - T && X < L + T) {
+                        AccWalk wk{left0, 0};
+                        acc_advance(&wk, off, ke);
+                        if (wk.x == lim) {
+                            if (off > 0.0) --k1;
+                            else ++k0;
+                        }
+                    }
                 }
+            }
+            const long long width = fix32(right0) - fix32(left0);
+            auto at = [&](int k) { return XL + static_cast<long long>(k) * S; };
+            // starts a hair below 0 (a few lines at most, but of a ray along the edge)
+            auto one = [&](int k) { sum += dd_line(I + k * w, at(k), at(k) + width, n); };
+            while (k0 <= k1 && at(k0) < 0) one(k0++);
+            while (k0 <= k1 && at(k1) < 0) one(k1--);
+            xl = at(k0);
+            xr = xl + width;
+        }
+    }
+    const bool any = k0 <= k1;
+    if (!any) xl = xr = S = 0;  // reads the first pixels of a line where the others are in step
+    // The last start whose footprint ends inside the image, with a margin for
+    // the FP32 right edge (within 3e-7 of the fixed-point one).
+    const long long last = (static_cast<long long>(n - 1) << 32) - 4096 - (xr - xl);
+    const long long span = xr - xl;
+    const float width = static_cast<float>(span) * 2.3283064365386963e-10f;  // 2^-32
+    const bool wide = __any_sync(0xffffffffu, any && !(width >= 0.001f && width <= 2.0f));
+    const float ends = sum;
+    const long long start = xl;
+    float acc = 0.0f;  // in units of half the width
+    // A line's four pixels are loaded whether its footprint reaches them or not
+    // (the copies have three zeros behind each line), and get the weight 0 where
+    // it does not: a ray that an infinity or NaN reached this way is summed
+    // again below.
+    auto step = [&](const float* __restrict__ line) {
+        const float* p = line + static_cast<int>(xl >> 32);
+        const float p0 = __ldg(p), p1 = __ldg(p + 1), p2 = __ldg(p + 2), p3 = __ldg(p + 3);
+        const float a = __uint_as_float(0x3F800000u | (static_cast<unsigned>(xl) >> 9));  // 1 + the start's fraction
+        const float e = a + width;
+        acc = fmaf(fminf(e, 2.0f) - a, p0 + p1, acc);
+        acc = fmaf(__saturatef(e - 2.0f), p1 + p2, acc);
+        acc = fmaf(__saturatef(e - 3.0f), p2 + p3, acc);
+        xl += S;
+    };
+    // the same for a line that some of the warp's rays may not have, and where
+    // the image may end inside the footprint (the start may sit a hair past
+    // n-1, where the exact one is inside)
+    auto step_edge = [&](const float* __restrict__ line, int l) {
+        const bool on = l >= k0 && l <= k1;
+        const int h = static_cast<int>(xl >> 32), i0 = max(min(h, n - 2), 0);
+        const float* p = line + i0;
+        const float p0 = __ldg(p), p1 = __ldg(p + 1), p2 = __ldg(p + 2), p3 = __ldg(p + 3);
+        const float a = h == i0 ? 1.0f + dd_frac(xl) : 2.0f;
+        const float e = fminf(a + width, static_cast<float>(n - i0));
+        float t = (fminf(e, 2.0f) - a) * (p0 + p1);
+        t = fmaf(__saturatef(e - 2.0f), p1 + p2, t);
+        t = fmaf(__saturatef(e - 3.0f), p2 + p3, t);
+        t = e > a ? __fdividef(t, e - a) : p0 + p1;
+        sum += on ? 0.5f * t : 0.0f;
+        xl += on ? S : 0;
+    };
+    // the lines of any ray of the warp, and those that all its rays have
+    const int lo = __reduce_min_sync(0xffffffffu, any ? k0 : 0x7fffffff);
+    const int hi = __reduce_max_sync(0xffffffffu, any ? k1 : -1);
+    const int in = __reduce_max_sync(0xffffffffu, any ? k0 : -1);
+    const int out = __reduce_min_sync(0xffffffffu, any ? k1 : 0x7fffffff);
+    const float* line = I + (lo <= hi ? lo : 0) * w;
+    const long long ahead = (kDdUnroll - 1) * S;
+    if (wide) {
+        for (int l = k0; l <= k1; ++l, xl += S) sum += dd_line(I + l * w, xl, xl + span, n);
+    } else {
+        for (int l = lo; l <= hi; l += kDdUnroll, line += kDdUnroll * w) {
+            if (l >= in && l + kDdUnroll - 1 <= out && !__any_sync(0xffffffffu, xl > last || xl + ahead > last)) {
+#pragma unroll
+                for (int u = 0; u < kDdUnroll; ++u) step(line + u * w);
+            } else {  // lines past the last one read the last one
+#pragma unroll
+                for (int u = 0; u < kDdUnroll; ++u) step_edge(l + u <= hi ? line + u * w : line, l + u);
             }
         }
     }
-    const float* I = (ux ? img : imgT) + blockIdx.y * img_stride;  // lines are rows of I
-    const long long XR = fix32(right0) + (XL - fix32(left0));        // the same anchor as the left edge
-    long long xl = XL + static_cast<long long>(k0) * S, xr = XR + static_cast<long long>(k0) * S;
-    float sum = 0.0f;
-    for (int l = k0; l <= k1; ++l) {
-        const int h = static_cast<int>(xl >> 32);
-        const int i0 = min(max(h, 0), n - 2);
-        // the start relative to interval i0 (clamped: the fixed-point start may
-        // sit a hair outside [0, n-1) where the exact one is inside)
-        const float lr = h == i0 ? dd_frac(xl) : (h < 0 ? 0.0f : 1.0f);
-        const int hr = static_cast<int>(xr >> 32);
-        const float rr = static_cast<float>(hr - i0) + dd_frac(xr);
-        const int ie = min(hr + (static_cast<unsigned>(xr) != 0u ? 1 : 0), n - 1);
-        const float* line = I + static_cast<size_t>(l) * n;
-        float tsum = 0.0f, lsum = 0.0f;
-        for (int i = i0; i < ie; ++i) {
-            const float j = static_cast<float>(i - i0);
-            const float len = fmaxf(fminf(j + 1.0f, rr) - fmaxf(j, lr), 0.0f);
-            tsum = fmaf(len, (__ldg(line + i) + __ldg(line + i + 1)) * 0.5f, tsum);
-            lsum += len;
+    if (is < ns) {
+        const float length = static_cast<float>(ux ? fabs(dy / sincos[2 * ia + 1]) : fabs(dx / sincos[2 * ia]));
+        if (any && !wide) {
+            sum += acc * (0.5f / width);
+            if (!isfinite(sum)) {
+                sum = ends;
+                xl = start;
+                for (int l = k0; l <= k1; ++l, xl += S) sum += dd_line(I + l * w, xl, xl + span, n);
+            }
         }
-        // a counted line always covers part of interval i0; where the clamped
-        // fixed-point edges leave no length, that sliver's trapezoid is the mean
-        sum += lsum > 0.0f ? tsum / lsum : (__ldg(line + i0) + __ldg(line + i0 + 1)) * 0.5f;
-        xl += S;
-        xr += S;
+        proj[blockIdx.y * proj_stride + ray] = sum * length;
     }
-    *out = sum * w;
 }
 
 // The reference's distance-driven grad in FP64 (T = double), one thread per
@@ -386,6 +485,324 @@ __global__ void __launch_bounds__(kDdThreads)
     img[blockIdx.y * img_stride + pix] = sum;
 }
 
+// ---- FP32 grad by tiles --------------------------------------------------------
+// A pixel-view's term is the integral over [x - o, x + o] (x the pixel's
+// position, o the view's |offset|) of the sinogram row read as cells of width 1
+// around the channels, halved and weighted.  As a function of x it is linear
+// between the positions where an end crosses from cell to cell: two knots a
+// channel.  So per (tile, view) the window of channels that the tile reaches is
+// staged once as those linear pieces, each from the few cells it covers, and a
+// pixel-view is one lookup and one FMA, whatever number of channels it covers.
+// With y = x + o - 1/2, j = floor(y) and f = y - j, the right end lies in cell
+// j + 1; with m = floor(2 o) and g = 2 o - m, the left end lies in cell j - m
+// where f < g, else in cell j - m + 1, and the integral is
+//   p[j-m+1] + ... + p[j] + g p[left] + f (p[j+1] - p[left]).
+// It is continuous in x, so the position needs no exact decision: it is FP32
+// relative to the window's centre, from the tile's 32.32 fixed-point reference.
+// Two things of the reference are decided: channels past the row's end read on
+// into the next view's row (the staging reads on likewise), and a footprint
+// that starts at or before -1/2 adds nothing (tiles that reach there test it
+// per pixel, in FP64 within 1e-3 of it).  Pixels at the ends of their line have
+// one-sided footprints: dd_grad_border sums those and overwrites them.
+//
+// CTA: 32 x 64 pixels, 8 of one column per thread, a segment of the views in
+// blocks of kDgViews; the next block's channels are loaded into registers
+// during a block's sums.  Bound by issue (72 % of the slots) and shared loads
+// (69 % of their wavefronts): 720 x 729 -> 512^2 1404 us pixel by pixel
+// (fp_dd_grad_f32), 147 us here (185 us with the views, border and sum
+// kernels).  A running integral over the window, looked up at both ends, took
+// as long and lost the digits of small channels beside a large one.
+constexpr int kDgTileX = 32, kDgTileY = 64, kDgRows = 8, kDgViews = 16, kDgThreads = 256;
+constexpr int kDgHalf = 64;  // channels staged on either side of the window's centre
+constexpr float kDgMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer in the low bits
+
+// A view's positions: channel of pixel (along, line) = b + along * o + line * l.
+struct DdView {
+    long long b, o, l;  // 32.32 fixed point
+    float of, lf;       // o and l
+    float half_w;       // half the view's weight
+    int flags;          // kDgUx: lines are rows; kDgBad: not of this form, or out of range
+};
+constexpr int kDgUx = 1, kDgBad = 2;
+
+// One warp per view, from the reference's (begin, offset) table of its lines.
+__global__ void __launch_bounds__(256)
+    dd_grad_views(const double* __restrict__ pos, const double* __restrict__ weights, const int* __restrict__ usex,
+                  DdView* __restrict__ views, int na, int n)
+{
+    const int ia = static_cast<int>((blockIdx.x * 256u + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (ia >= na) return;
+    const double* pp = pos + static_cast<size_t>(ia) * n * 2;
+    const double b = pp[0], o = pp[1], l = n > 1 ? (pp[2 * (n - 1)] - b) / (n - 1) : 0.0;
+    bool ok = fabs(b) < 1048576.0 && fabs(o) < 1048576.0 && fabs(l) < 1048576.0 &&
+              fabs(o) * n < 1e9 && fabs(l) * n < 1e9;
+    for (int i = lane; i < n; i += 32)
+        ok = ok && pp[2 * i + 1] == o && fabs(pp[2 * i] - fma(static_cast<double>(i), l, b)) < 1e-8;
+    ok = __all_sync(0xffffffffu, ok);
+    if (lane == 0)
+        views[ia] = DdView{ok ? fix32(b) : 0, ok ? fix32(o) : 0, ok ? fix32(l) : 0, static_cast<float>(o),
+                           static_cast<float>(l), 0.5f * static_cast<float>(weights[ia]), (usex[ia] ? kDgUx : 0) | (ok ? 0 : kDgBad)};
+}
+
+// A view on a tile.
+enum DgMode { kDgSkip, kDgInside, kDgEdge, kDgSlow };
+struct DgRec {
+    float base, sx, sy;  // y - 1/2 of the tile's reference pixel, relative to the window's centre, and its slopes
+    float knot;          // g - 1/2
+    float limit;         // footprints with y - 1/2 at or below it add nothing
+    int mode;
+    float reach;  // o
+    int flags;    // the view's
+};
+
+__device__ __forceinline__ DgRec dg_record(const DdView& v, int tx0, int ty0, int* centre, int* need)
+{
+    const bool ux = v.flags & kDgUx;
+    // the reference pixel (the tile's centre); it may lie outside the image
+    const long long cx = tx0 + kDgTileX / 2, cy = ty0 + kDgTileY / 2;
+    const long long mid = v.b + (ux ? cx : cy) * v.o + (ux ? cy : cx) * v.l;
+    const long long kc = (mid + kDdHalf) >> 32;
+    DgRec r;
+    r.sx = ux ? v.of : v.lf;
+    r.sy = ux ? v.lf : v.of;
+    r.reach = fabsf(v.of);
+    r.base = static_cast<float>(static_cast<int>(mid)) * 2.3283064365386963e-10f + (r.reach - 1.0f);  // mid - kc
+    r.knot = 2.0f * r.reach - floorf(2.0f * r.reach) - 0.5f;
+    r.flags = v.flags;
+    // positions of the tile lie within e of the centre
+    const float e = fabsf(r.sx) * (kDgTileX / 2) + fabsf(r.sy) * (kDgTileY / 2) + 0.51f;
+    const float start = -0.5f - fmaxf(fminf(static_cast<float>(kc), 1e6f), -1e6f);  // channel -1/2, from the centre
+    r.limit = start + (2.0f * r.reach - 1.0f);
+    if ((v.flags & kDgBad) || !(e + r.reach < kDgHalf - 3) || kc <= -1000000 || kc >= 0x40000000)
+        r.mode = kDgSlow;
+    else if (e < start - 0.01f)
+        r.mode = kDgSkip;
+    else
+        r.mode = -e - r.reach > start + 0.01f ? kDgInside : kDgEdge;
+    *centre = static_cast<int>(kc);
+    *need = r.mode == kDgInside || r.mode == kDgEdge ? static_cast<int>(e + r.reach) + 2 : -1;
+    return r;
+}
+
+__global__ void __launch_bounds__(kDgThreads, 3)
+    dd_grad_tiles(const float* __restrict__ proj, float* __restrict__ out, const double* __restrict__ pos,
+                  const DdView* __restrict__ views, int ns, int na, int n, int segs, int seg_len, size_t out_seg,
+                  size_t out_img)
+{
+    constexpr unsigned kSecond = 2 * kDgHalf * sizeof(float2);  // from a piece before the knot to the one after it
+    __shared__ __align__(16) float2 s_piece[kDgViews][2][2 * kDgHalf];
+    __shared__ __align__(16) float s_row[8][2 * kDgHalf + 4];  // a warp's channels while it forms the pieces
+    __shared__ DgRec s_rec[kDgViews];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tx0 = blockIdx.x * kDgTileX, ty0 = blockIdx.y * kDgTileY;
+    const int seg = blockIdx.z % segs, b = blockIdx.z / segs;
+    const int vb = seg * seg_len, ve = min(na, vb + seg_len);
+    const long long total = static_cast<long long>(na) * ns;
+    const float* P = proj + b * static_cast<size_t>(total);
+    const int ix = tx0 + lane, iy0 = ty0 + warp * kDgRows;
+    const float ox = static_cast<float>(lane - kDgTileX / 2), oy = static_cast<float>(warp * kDgRows - kDgTileY / 2);
+
+    // staging: a warp takes views warp and warp + 8 of a block, four channels a lane
+    constexpr int kPer = kDgViews / 8;
+    static_assert(2 * kDgHalf == 4 * 32 && kDgThreads == 256, "four channels a lane, eight warps");
+    float4 ch[kPer];
+    DgRec rec[kPer];
+    int need[kPer];
+    auto load = [&](int v0) {
+#pragma unroll
+        for (int h = 0; h < kPer; ++h) {
+            const int ia = v0 + warp + 8 * h;
+            if (ia >= ve) continue;
+            const DdView v = views[ia];
+            int kc;
+            rec[h] = dg_record(v, tx0, ty0, &kc, &need[h]);
+            const long long row = static_cast<long long>(ia) * ns, room = min(total - row, 0x7fffffffll);
+            auto one = [&](int i) {
+                const int rel = 4 * lane + i - kDgHalf, c = kc + rel;
+                return abs(rel) <= need[h] && c >= 0 && c < static_cast<int>(room) ? __ldg(P + row + c) * v.half_w : 0.0f;
+            };
+            ch[h] = make_float4(one(0), one(1), one(2), one(3));
+        }
+    };
+    auto stage = [&](int v0) {
+#pragma unroll
+        for (int h = 0; h < kPer; ++h) {
+            const int j = warp + 8 * h;
+            if (v0 + j >= ve) continue;
+            float* row = s_row[warp];
+            __syncwarp();
+            reinterpret_cast<float4*>(row)[lane] = ch[h];
+            if (lane == 0) row[2 * kDgHalf] = 0.0f;
+            __syncwarp();
+            const float two = 2.0f * rec[h].reach;
+            const int m = static_cast<int>(fminf(two, 2.0f * kDgHalf));
+            const float g = two - static_cast<float>(m);
+            // the pieces that the tile's positions can fall in
+            for (int i = kDgHalf - need[h] + lane; i < kDgHalf + need[h]; i += 32) {
+                const float right = row[i + 1], after = row[i - m + 1], before = row[max(i - m, 0)];
+                float sum = m > 0 ? row[i] : 0.0f;
+                if (m > 1) sum += after;
+                for (int k = i - m + 2; k < i; ++k) sum += row[k];
+                const float sa = right - before, sb = right - after;
+                s_piece[j][0][i] = make_float2(fmaf(0.5f, sa, fmaf(g, before, sum)), sa);  // from f = 1/2
+                s_piece[j][1][i] = make_float2(fmaf(0.5f, sb, fmaf(g, after, sum)), sb);
+            }
+            if (lane == 0) s_rec[j] = rec[h];
+        }
+    };
+
+    const unsigned pieces = static_cast<unsigned>(__cvta_generic_to_shared(&s_piece[0][0][kDgHalf])) -
+                            (__float_as_uint(kDgMagic) << 3);
+    float acc[kDgRows] = {};
+    load(vb);
+    for (int v0 = vb; v0 < ve; v0 += kDgViews) {
+        const int nv = min(kDgViews, ve - v0);
+        stage(v0);
+        __syncthreads();
+        load(v0 + kDgViews);
+        float blk[kDgRows] = {};  // this block's sums
+        for (int j = 0; j < nv; ++j) {
+            const DgRec r = s_rec[j];
+            if (r.mode == kDgSkip) continue;
+            if (r.mode == kDgSlow) {
+                const long long row = static_cast<long long>(v0 + j) * ns;
+                const bool ux = r.flags & kDgUx;
+                for (int k = 0; k < kDgRows; ++k) {
+                    const int iy = iy0 + k;
+                    int first, cnt;
+                    float lr, rr, t = 0.0f;
+                    if (ix < n && iy < n &&
+                        dd_grad_decide64(pos + static_cast<size_t>(v0 + j) * n * 2, ux, ix, iy, n, n, total - 1 - row,
+                                         first, cnt, lr, rr))
+                        for (int c = 0; c < cnt; ++c) {
+                            const float fc = static_cast<float>(c);
+                            const float len = fminf(fc + 0.5f, rr) - fmaxf(fc - 0.5f, lr);
+                            t = fmaf(len, __ldg(P + row + first + c), t);
+                        }
+#pragma unroll
+                    for (int q = 0; q < kDgRows; ++q)  // blk stays in registers
+                        if (q == k) blk[q] = fmaf(t, views[v0 + j].half_w, blk[q]);
+                }
+                continue;
+            }
+            const unsigned at = pieces + j * static_cast<unsigned>(sizeof s_piece[0]), at2 = at + kSecond;
+            const float xc = fmaf(ox, r.sx, r.base);
+            const float2 sy = make_float2(r.sy, r.sy), x0 = make_float2(xc, xc);
+            auto rows = [&](auto keep) {
+#pragma unroll
+                for (int k = 0; k < kDgRows; k += 2) {
+                    const float2 y = __ffma2_rn(make_float2(oy + k, oy + (k + 1)), sy, x0);
+                    const float2 t = __fadd2_rn(y, make_float2(kDgMagic, kDgMagic));
+                    const float2 f = __ffma2_rn(__fadd2_rn(t, make_float2(-kDgMagic, -kDgMagic)),
+                                                make_float2(-1.0f, -1.0f), y);
+                    float2 p, q;
+                    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
+                                 : "=f"(p.x), "=f"(p.y) : "r"((f.x < r.knot ? at : at2) + (__float_as_uint(t.x) << 3)));
+                    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
+                                 : "=f"(q.x), "=f"(q.y) : "r"((f.y < r.knot ? at : at2) + (__float_as_uint(t.y) << 3)));
+                    keep(y, k, p, q);
+                    blk[k] += fmaf(f.x, p.y, p.x);
+                    blk[k + 1] += fmaf(f.y, q.y, q.x);
+                }
+            };
+            if (r.mode == kDgInside) {
+                rows([](float2, int, float2&, float2&) {});
+            } else {  // footprints that start before the first channel are left out
+                rows([&](float2 y, int k, float2& p, float2& q) {
+                    auto on = [&](float yk, int iy) {
+                        if (fabsf(yk - r.limit) < 1e-3f && ix < n && iy < n) {
+                            int first, cnt;
+                            float lr, rr;
+                            return dd_grad_decide64(pos + static_cast<size_t>(v0 + j) * n * 2, r.flags & kDgUx, ix, iy,
+                                                    n, n, total - 1 - static_cast<long long>(v0 + j) * ns, first, cnt,
+                                                    lr, rr);
+                        }
+                        return yk > r.limit;
+                    };
+                    if (!on(y.x, iy0 + k)) p = make_float2(0.0f, 0.0f);
+                    if (!on(y.y, iy0 + k + 1)) q = make_float2(0.0f, 0.0f);
+                });
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kDgRows; ++k) acc[k] += blk[k];
+        __syncthreads();
+    }
+    float* O = out + seg * out_seg + b * out_img;
+#pragma unroll
+    for (int k = 0; k < kDgRows; ++k)
+        if (ix < n && iy0 + k < n) O[static_cast<size_t>(iy0 + k) * n + ix] = acc[k];
+}
+
+// The 4n - 4 pixels at the image's border, overwriting dd_grad_tiles' values: a
+// warp takes 32 adjacent pixels of one side and every 32nd view, so that its
+// loads are adjacent channels of a row, and the block's warps are added in a
+// fixed order.  Their footprints are one-sided where the pixel ends its line.
+constexpr int kDbThreads = 1024;
+__global__ void __launch_bounds__(kDbThreads)
+    dd_grad_border(const float* __restrict__ proj, float* __restrict__ img, const double* __restrict__ pos,
+                   const DdView* __restrict__ views, int ns, int na, int n, int groups)
+{
+    __shared__ float s_sum[kDbThreads / 32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int side = blockIdx.x / groups, i = (blockIdx.x - side * groups) * 32 + lane;
+    const int end = side & 1 ? n - 1 : 0;
+    const int ix = side < 2 ? min(i, n - 1) : end, iy = side < 2 ? end : min(i, n - 1);
+    const long long total = static_cast<long long>(na) * ns;
+    const float* P = proj + blockIdx.y * static_cast<size_t>(total);
+    float sum = 0.0f;
+    for (int ia = warp; ia < na; ia += kDbThreads / 32) {
+        const DdView v = views[ia];
+        const bool ux = v.flags & kDgUx;
+        const int along = ux ? ix : iy, line = ux ? iy : ix;
+        const long long row = static_cast<long long>(ia) * ns;
+        const long long mid = v.b + along * v.o + line * v.l;
+        long long left = along == 0 ? mid : mid - v.o, right = along == n - 1 ? mid : mid + v.o;
+        if (left > right) {
+            const long long t = left;
+            left = right;
+            right = t;
+        }
+        const long long c = (left + kDdHalf) >> 32;  // the left end's cell
+        int first = static_cast<int>(c), cnt = static_cast<int>(((right + kDdHalf) >> 32) - c) + 1;
+        float lr = static_cast<float>(left - (c << 32)) * 2.3283064365386963e-10f;
+        float rr = static_cast<float>(right - (c << 32)) * 2.3283064365386963e-10f;
+        const long long past = left + kDdHalf;  // > 0: the view counts (tie: decided in FP64)
+        bool on = past > 0;
+        if ((v.flags & kDgBad) || (past > -(1ll << 16) && past < (1ll << 16)))
+            on = dd_grad_decide64(pos + static_cast<size_t>(ia) * n * 2, ux, ix, iy, n, n, total - 1 - row, first, cnt,
+                                  lr, rr);
+        if (!on) continue;
+        float t = 0.0f;
+        for (int k = 0; k < cnt; ++k) {
+            const long long at = row + first + k;
+            const float fk = static_cast<float>(k);
+            const float len = fminf(fk + 0.5f, rr) - fmaxf(fk - 0.5f, lr);
+            if (first + k >= 0 && at < total) t = fmaf(len, __ldg(P + at), t);
+        }
+        sum = fmaf(t, v.half_w, sum);
+    }
+    s_sum[warp][lane] = sum;
+    __syncthreads();
+    if (warp == 0 && i < n) {
+        float a = s_sum[0][lane];
+#pragma unroll
+        for (int k = 1; k < kDbThreads / 32; ++k) a += s_sum[k][lane];
+        img[static_cast<size_t>(blockIdx.y) * n * n + static_cast<size_t>(iy) * n + ix] = a;
+    }
+}
+
+// img[e] = part[0][e] + part[1][e] + ... in segment order.
+__global__ void __launch_bounds__(256)
+    dd_grad_sum(const float* __restrict__ part, float* __restrict__ img, size_t count, int segs)
+{
+    for (size_t e = blockIdx.x * 256ull + threadIdx.x; e < count; e += gridDim.x * 256ull) {
+        float a = part[e];
+        for (int s = 1; s < segs; ++s) a += part[s * count + e];
+        img[e] = a;
+    }
+}
+
 int check_dd(const ctr_par_param* p, const void* a, const void* b, const void* t0, const void* t1,
              const void* t2, int batch)
 {
@@ -416,16 +833,72 @@ int dd_forward(const ctr_par_param* p, const T* img, T* proj, const double* sc, 
     } else {
         const int n = static_cast<int>(p->nx);
         if (batch > 65535) return fail(CTR_ERR_UNSUPPORTED, "batch > 65535");
-        float* imgT = nullptr;
-        cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&imgT), sizeof(float) * is * batch, stream);
+        float* rows = nullptr;
+        const size_t copy = static_cast<size_t>(n) * (n + kDdPad);
+        cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&rows), 2 * sizeof(float) * copy * batch, stream);
         if (e != cudaSuccess) return fail(CTR_ERR_CUDA, "distance-driven scratch: %s", cudaGetErrorString(e));
-        dd_transpose<<<dim3(div_up(n, 32), div_up(n, 32), batch), 256, 0, stream>>>(img, imgT, n);
-        fp_dd_f32<<<grid, kDdThreads, 0, stream>>>(img, imgT, proj, sc, bo, usex, p->ns, p->na, n, p->dx, p->dy,
-                                                   is, ps);
+        float* cols = rows + copy * batch;
+        const unsigned tiles = div_up(n + kDdPad, 32), chunks = div_up(p->ns, kDdRayThreads);
+        dd_copies<<<dim3(tiles, tiles, batch), 256, 0, stream>>>(img, rows, cols, n);
+        fp_dd_f32<<<dim3(chunks * p->na, batch), kDdRayThreads, 0, stream>>>(
+            img, rows, cols, proj, sc, bo, usex, p->ns, chunks, n, p->dx, p->dy, is, ps);
         st = check_launch("fp_par_2d distance driven");
-        cudaFreeAsync(imgT, stream);  // after the kernel that reads it
+        cudaFreeAsync(rows, stream);  // after the kernel that reads it
         return st;
     }
+}
+
+constexpr int kDgNotTiles = -1;
+
+// The grad by tiles, kDgNotTiles where a tile's channels do not fit its window
+// (pixels of more than ~1.6 channels): those calls run pixel by pixel.  By
+// tiles is the faster one wherever it can run: 512^2 x 720 x 729 185 us against
+// 1415, 64^2 x 90 x 96 40 against 76.
+int dd_grad_by_tiles(const ctr_par_param* p, const float* proj, float* img, const double* w, const double* pos,
+                     const int* usex, int batch, cudaStream_t stream)
+{
+    const int n = static_cast<int>(p->nx), na = static_cast<int>(p->na);
+    const double reach = std::hypot(kDgTileX / 2 * p->dx, kDgTileY / 2 * p->dy) + std::fmax(std::fabs(p->dx), std::fabs(p->dy));
+    if (!(reach / std::fabs(p->ds) < kDgHalf - 4)) return kDgNotTiles;
+    const int tiles_x = div_up(n, kDgTileX), tiles_y = div_up(n, kDgTileY);
+    const long long tiles = static_cast<long long>(tiles_x) * tiles_y;
+    // Segments of the views per tile, for the fewest view blocks on the busiest
+    // SM (three CTAs a SM).  A function of the geometry and device only, so an
+    // image's sums are the same in any batch.
+    const int blocks = div_up(na, kDgViews), slots = 3 * device_sms();
+    int segs = 1, len = blocks;
+    long long best = (tiles + slots - 1) / slots * blocks;
+    for (int s = 2; s <= 16 && s <= blocks; ++s) {
+        const int l = div_up(blocks, s), used = div_up(blocks, l);
+        const long long cost = (tiles * used + slots - 1) / slots * l;
+        if (cost < best) {
+            best = cost;
+            segs = used;
+            len = l;
+        }
+    }
+    if (tiles_y > 65535 || static_cast<long long>(segs) * batch > 65535) return kDgNotTiles;
+    const size_t image = static_cast<size_t>(n) * n, count = image * batch;
+    const size_t part_at = (sizeof(DdView) * na + 255) / 256 * 256;
+    char* scratch = nullptr;
+    if (cudaMallocAsync(reinterpret_cast<void**>(&scratch), part_at + (segs > 1 ? sizeof(float) * segs * count : 0),
+                        stream) != cudaSuccess) {
+        cudaGetLastError();  // no room for the partial images
+        return kDgNotTiles;
+    }
+    DdView* views = reinterpret_cast<DdView*>(scratch);
+    float* part = segs > 1 ? reinterpret_cast<float*>(scratch + part_at) : img;
+    dd_grad_views<<<div_up(na, 8), 256, 0, stream>>>(pos, w, usex, views, na, n);
+    dd_grad_tiles<<<dim3(tiles_x, tiles_y, segs * batch), kDgThreads, 0, stream>>>(
+        proj, part, pos, views, static_cast<int>(p->ns), na, n, segs, len * kDgViews, count, image);
+    if (segs > 1)
+        dd_grad_sum<<<std::min<size_t>(div_up(count, 256), 8u * device_sms()), 256, 0, stream>>>(part, img, count, segs);
+    const int groups = div_up(n, 32);
+    dd_grad_border<<<dim3(4 * groups, batch), kDbThreads, 0, stream>>>(proj, img, pos, views, static_cast<int>(p->ns),
+                                                                       na, n, groups);
+    const int st = check_launch("fp_par_2d distance-driven grad");
+    cudaFreeAsync(scratch, stream);  // after the kernels that read it
+    return st;
 }
 
 template <typename T>
@@ -441,6 +914,8 @@ int dd_grad(const ctr_par_param* p, const T* proj, T* img, const double* w, cons
             static_cast<size_t>(p->na) * p->ns);
         return check_launch("fp_par_2d distance-driven grad");
     } else {
+        const int rc = dd_grad_by_tiles(p, proj, img, w, pos, usex, batch, stream);
+        if (rc != kDgNotTiles) return rc;
         // the fixed-point table and FP32 weights of this call (stream-ordered scratch)
         const size_t n_fx = static_cast<size_t>(p->na) * p->nx;
         char* scratch = nullptr;
