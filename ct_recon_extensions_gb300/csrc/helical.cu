@@ -9,7 +9,7 @@
 // cos(gamma) and per-slice view ranges come from the host
 // (ctr_helical_interpolation_prep) with the reference's own libm calls, so the
 // output equals the reference's bit for bit.  T=float runs the FP32 fast path
-// (helical_fast_f32): the same decisions as the reference (rows, usability,
+// (helical_360_f32, helical_fast_f32): the same decisions as the reference (rows, usability,
 // views) with FP32 sums, falling back to the exact computation per sample
 // where an FP32 decision could differ; GB300's FP64 rate is 1/64 of its FP32
 // rate, which made the exact kernel compute-bound at <1 % of HBM bandwidth.
@@ -457,6 +457,251 @@ __global__ void __launch_bounds__(kHeliThreads, M == CTR_HELICAL_360 ? 8 : 6)
         heli_fast_one<M>(in, o + static_cast<size_t>(iv) * g.ns, tab, g, s, rows[iv], cf, iv, is, status);
 }
 
+// ---- 360LI, FP32: rows decided once per 32 channels ----------------------------
+// Along a row of channels cos(gamma) changes slowly, so over 32 channels a slab
+// edge lies in one or two cells of the detector rows.  A warp takes 32 channels
+// of kH3Views views x kH3Slices slices: lane t first decides task t (one view of
+// one slice) for all its channels from the extremes of cos(gamma) over them, the
+// ends of an edge's range away from integers by the guard of near_int.  Then the
+// warp takes the tasks one by one.  Where both edges stay in one cell a task is
+// a few coalesced row loads and one multiplication a sample.  Where an edge
+// passes from a cell to the next, each lane compares its edge with the one
+// integer between them (lanes within the guard of it send the task to
+// heli_fast_one, as do the tasks at the detector's ends).  The slices of a view
+// follow one another, since the slabs of neighbouring slices share most of
+// their rows (L1).  Latency and issue bound: a scan of 128 slices x 1152 views x
+// 736 channels takes 340 us, 858 us sample by sample (157 -> 73 instructions a
+// sample).  The samples left in a second kernel, from a list in scratch: 413 us;
+// besides that, branches in place of the predicated loads 450 us, one task at a
+// time in order 543 us, 8 blocks an SM (63 registers) 501 us.
+constexpr int kH3Views = 4, kH3Slices = 8, kH3Warps = 4, kH3Group = 2;
+static_assert(kH3Views * kH3Slices == 32, "a task a lane");
+
+// *p where n > K (x < 0), else 0: predicated loads, where a branch would wait for
+// each load before the next is issued.
+template <int K>
+__device__ __forceinline__ float ldg_above(const float* p, int n)
+{
+    float v;
+    asm("{\n\t.reg .pred q;\n\tsetp.gt.s32 q, %2, %3;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}"
+        : "=f"(v)
+        : "l"(p), "r"(n), "n"(K));
+    return v;
+}
+__device__ __forceinline__ float ldg_negative(const float* p, float x)
+{
+    float v;
+    asm("{\n\t.reg .pred q;\n\tsetp.lt.f32 q, %2, 0f00000000;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}"
+        : "=f"(v)
+        : "l"(p), "f"(x));
+    return v;
+}
+
+// One edge of a slab over the channels: the rows that all of them use start (top)
+// or end (bottom) at row `all`; a lane's edge lies k - a g past the integer
+// `all` (k = 1 or -1 and a = 0 where no lane's lies on its other side).
+struct H3Edge {
+    float k, a;
+    int all;
+    bool sure;
+};
+
+enum H3Kind { kH3None, kH3Rows, kH3Mixed, kH3Two, kH3Slow };
+// One sample's rows for all channels: `at` the element of the first row that all
+// of them use (channel 0), n rows; w the z weight (kH3Rows: over n); the output
+// element of channel 0; the edges.
+struct H3View {
+    unsigned at;
+    int n;
+    float w;
+    unsigned out;
+    float tk, ta, bk, ba;
+};
+static_assert(sizeof(H3View) == 32, "16-byte loads");
+
+__device__ __forceinline__ H3Edge h3_edge(const HeliGeo& g, float a, float g0, float g1, float guard, bool top)
+{
+    const float x0 = g.ct_f - a * g0, x1 = g.ct_f - a * g1;
+    const float lo = fminf(x0, x1), hi = fmaxf(x0, x1), fl = floorf(lo), fh = floorf(hi);
+    // all edges clamped to the detector's end: floor(max(x, 0)) = 0, ceil(min(x, nt)) = nt
+    const bool clamped = top ? hi < 1.0f - guard : lo > g.nt_f - 1.0f + guard;
+    H3Edge e;
+    const bool away = lo - fl > guard && fh + 1.0f - hi > guard;
+    const bool two = !clamped && fh == fl + 1.0f;
+    e.sure = clamped || (away && (fh == fl || two));
+    const float row = top ? (clamped ? 0.0f : fh) : (clamped ? g.nt_f : (two ? fh : fl + 1.0f));
+    e.all = static_cast<int>(row);
+    e.k = two ? g.ct_f - row : (top ? 1.0f : -1.0f);
+    e.a = two ? a : 0.0f;
+    return e;
+}
+
+// The rows of one sample's slab with the quotients a (top) and b (bottom):
+// false where they are left to heli_fast_one; n = 0 and no edge where it misses.
+__device__ __forceinline__ bool h3_rows(const HeliGeo& g, float a, float b, float g0, float g1, float guard, H3Edge& t,
+                                        H3Edge& e)
+{
+    t = e = H3Edge{0.0f, 0.0f, 0, true};
+    t.k = 1.0f;
+    e.k = -1.0f;
+    const float b0 = g.ct_f - b * g0, b1 = g.ct_f - b * g1, t0 = g.ct_f - a * g0, t1 = g.ct_f - a * g1;
+    if (fmaxf(b0, b1) < -guard || fminf(t0, t1) >= g.nt_f + guard) return true;  // misses for every channel
+    if (fminf(b0, b1) <= guard || fmaxf(t0, t1) >= g.nt_f - guard) return false;
+    t = h3_edge(g, a, g0, g1, guard, true);
+    e = h3_edge(g, b, g0, g1, guard, false);
+    return t.sure && e.sure && e.all >= t.all;
+}
+
+// A sample that its task left.  Out of line: its registers would halve the
+// kernel's blocks an SM.
+__device__ __noinline__ void h3_slow(const float* in, float* out, const HeliHeader* tab, const HeliGeo& g,
+                                     unsigned* status, unsigned iz, unsigned iv, unsigned is)
+{
+    const HeliSlice* slices = heli_slices<CTR_HELICAL_360>(tab, g);
+    const HeliChanF cf = reinterpret_cast<const HeliChanF*>(slices + g.nz)[is];
+    const size_t row = static_cast<size_t>(iz) * g.vpr + iv;
+    heli_fast_one<CTR_HELICAL_360>(in, out + row * g.ns + is, tab, g, slices[iz],
+                                   heli_rows_f<CTR_HELICAL_360>(tab, g)[row], cf, iv, is, status + iz);
+}
+
+__global__ void __launch_bounds__(32 * kH3Warps, 12)
+    helical_360_f32(const float* __restrict__ in, float* __restrict__ out, const HeliHeader* __restrict__ tab,
+                    const __grid_constant__ HeliGeo g, unsigned* status, int slice_groups, unsigned chunks)
+{
+    __shared__ __align__(16) H3View s_view[2][kH3Warps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned b = blockIdx.z / slice_groups, group = blockIdx.z - b * slice_groups, iz0 = group * kH3Slices;
+    const unsigned chunk = blockIdx.x * kH3Warps + warp, c0 = chunk * 32;
+    if (chunk >= chunks) return;  // warp-uniform
+    const unsigned is = min(c0 + lane, g.ns - 1);
+    in += b * g.in_item;
+    out += b * g.out_item;
+    status += b * g.nz;
+    if (tab->method != CTR_HELICAL_360 || tab->ns != g.ns || tab->nz != g.nz || tab->vpr != g.vpr) {
+        if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && iz0 == 0) atomicOr(status, CTR_HELICAL_BAD_TABLE);
+        return;
+    }
+    const HeliSlice* slices = heli_slices<CTR_HELICAL_360>(tab, g);
+    const float gc = reinterpret_cast<const HeliChanF*>(slices + g.nz)[is].g;
+    const HeliRowF* rows = heli_rows_f<CTR_HELICAL_360>(tab, g);
+    float g0 = gc, g1 = gc;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        g0 = fminf(g0, __shfl_xor_sync(0xffffffffu, g0, o));
+        g1 = fmaxf(g1, __shfl_xor_sync(0xffffffffu, g1, o));
+    }
+    // near_int's guard for any edge on the detector (within one row of it)
+    const float guard = kEdgeGuard + (g.nt_f + 1.0f + fabsf(g.ct_f)) * kEdgeGuardRel;
+    const bool on = c0 + lane < g.ns;
+    const unsigned ns = g.ns;
+    const unsigned iz = iz0 + lane % kH3Slices;
+    bool valid = false;
+    if (iz < g.nz) {
+        valid = slices[iz].valid;
+        if (!valid && c0 == 0 && blockIdx.y == 0)  // the reference throws before touching this slice
+            atomicOr(status + iz, CTR_HELICAL_NO_VIEWS);
+    }
+    const unsigned iv = blockIdx.y * kH3Views + lane / kH3Slices;
+    int kind = kH3None;
+    if (valid && iv < g.vpr) {
+        const HeliRowF& r = rows[static_cast<size_t>(iz) * g.vpr + iv];
+        H3Edge t1, b1, t2, b2;
+        const bool sure = h3_rows(g, r.at, r.ab, g0, g1, guard, t1, b1) &&
+                          h3_rows(g, r.at2, r.ab2, g0, g1, guard, t2, b2);
+        const bool hit1 = b1.all > 0, hit2 = b2.all > 0;  // the last row's end
+        const bool mixed = t1.a != 0.0f || b1.a != 0.0f || t2.a != 0.0f || b2.a != 0.0f;
+        kind = !sure || !(hit1 || hit2) ? kH3Slow : hit1 && hit2 ? kH3Two : mixed ? kH3Mixed : kH3Rows;
+        auto view = [&](int i, int from, const H3Edge& top, const H3Edge& bot, float w) {
+            H3View v;
+            v.n = bot.all - top.all;
+            v.at = (static_cast<unsigned>(from) * g.nt + top.all) * g.ns;
+            v.w = kind == kH3Rows ? __fdividef(1.0f, static_cast<float>(v.n)) : w;
+            v.out = (iz * g.vpr + iv) * g.ns;
+            v.tk = top.k;
+            v.ta = top.a;
+            v.bk = bot.k;
+            v.ba = bot.a;
+            s_view[i][warp][lane] = v;
+        };
+        if (hit1) view(0, r.cur, t1, b1, hit2 ? r.wcur : 1.0f);
+        if (hit2) view(hit1 ? 1 : 0, r.cor, t2, b2, hit1 ? r.wcor : 1.0f);
+    }
+    unsigned m_rows = __ballot_sync(0xffffffffu, kind == kH3Rows);
+    unsigned m_mixed = __ballot_sync(0xffffffffu, kind == kH3Mixed);
+    unsigned m_two = __ballot_sync(0xffffffffu, kind == kH3Two);
+    unsigned slow = __ballot_sync(0xffffffffu, kind == kH3Slow);
+    __syncwarp();
+    // the next tasks of a class, the last one again where there are fewer (the
+    // repeated ones write the same value)
+    auto take = [](unsigned& m, int (&k)[kH3Group]) {
+#pragma unroll
+        for (int u = 0; u < kH3Group; ++u) {
+            k[u] = __ffs(m) - 1;
+            const unsigned rest = m & (m - 1);
+            if (u == kH3Group - 1 || rest) m = rest;
+        }
+    };
+    auto sum = [&](unsigned at, int n) {
+        float s = (ldg_above<0>(in + at, n) + ldg_above<1>(in + (at + ns), n)) +
+                  (ldg_above<2>(in + (at + 2 * ns), n) + ldg_above<3>(in + (at + 3 * ns), n));
+        for (int r = 4; r < n; ++r) s += __ldg(in + (at + r * ns));
+        return s;
+    };
+    // the mean of a lane's rows; near: a lane's edge is too close to the integer
+    auto mean = [&](const H3View& v, bool& near) {
+        const float dt = fmaf(-v.ta, gc, v.tk), db = fmaf(v.ba, gc, -v.bk);  // minus what b lies past its integer
+        near = near || fminf(fabsf(dt), fabsf(db)) < guard;
+        const unsigned at = v.at + is;
+        int n = v.n;
+        const float s = (ldg_negative(in + (at - ns), dt) + ldg_negative(in + (at + n * ns), db)) + sum(at, n);
+        n += (dt < 0.0f ? 1 : 0) + (db < 0.0f ? 1 : 0);
+        return __fdividef(s, static_cast<float>(n));
+    };
+    while (m_rows) {
+        int k[kH3Group];
+        take(m_rows, k);
+        float v[kH3Group];
+        unsigned to[kH3Group];
+#pragma unroll
+        for (int u = 0; u < kH3Group; ++u) {
+            const uint4 t = *reinterpret_cast<const uint4*>(&s_view[0][warp][k[u]]);
+            v[u] = __uint_as_float(t.z) * sum(t.x + is, static_cast<int>(t.y));
+            to[u] = t.w + is;
+        }
+#pragma unroll
+        for (int u = 0; u < kH3Group; ++u)
+            if (on) out[to[u]] = v[u];
+    }
+    while (m_mixed) {
+        int k[kH3Group];
+        take(m_mixed, k);
+        float v[kH3Group];
+        bool near[kH3Group];
+#pragma unroll
+        for (int u = 0; u < kH3Group; ++u) {
+            near[u] = false;
+            v[u] = mean(s_view[0][warp][k[u]], near[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < kH3Group; ++u) {
+            if (__any_sync(0xffffffffu, near[u])) slow |= 1u << k[u];
+            else if (on) out[s_view[0][warp][k[u]].out + is] = v[u];
+        }
+    }
+    for (; m_two; m_two &= m_two - 1) {
+        const int k = __ffs(m_two) - 1;
+        bool near = false;
+        const H3View a = s_view[0][warp][k], c = s_view[1][warp][k];
+        const float ma = mean(a, near), mc = mean(c, near);
+        if (__any_sync(0xffffffffu, near)) slow |= 1u << k;
+        else if (on) out[a.out + is] = fmaf(c.w, mc, a.w * ma);
+    }
+    for (; slow && on; slow &= slow - 1) {  // sample by sample
+        const int k = __ffs(slow) - 1;
+        h3_slow(in, out, tab, g, status, iz0 + k % kH3Slices, blockIdx.y * kH3Views + k / kH3Slices, is);
+    }
+}
+
 size_t table_bytes(const ctr_helical_param* p)
 {
     return sizeof(HeliHeader) + sizeof(HeliChan) * p->ns + sizeof(HeliSlice) * p->nz + sizeof(HeliChanF) * p->ns +
@@ -516,6 +761,19 @@ bool fast_ok(const ctr_helical_param* p)
            p->na < (1u << 20) && p->nt < (1u << 15) && std::fabs(p->view_per_rot * p->couch_mov) < 1e4;
 }
 
+// 360LI by tasks: false (nothing launched) where an item's elements need more
+// than 32 bits.
+bool launch_360(const ctr_helical_param* p, const HeliGeo& g, const float* in, float* out, const HeliHeader* tab,
+                unsigned* status, int batch, cudaStream_t stream)
+{
+    const unsigned chunks = div_up(p->ns, 32), views = div_up(p->view_per_rot, kH3Views),
+                   groups = div_up(p->nz, kH3Slices);
+    if (g.in_item > 0xffffffffu || g.out_item > 0xffffffffu) return false;
+    helical_360_f32<<<dim3(div_up(chunks, kH3Warps), views, groups * batch), 32 * kH3Warps, 0, stream>>>(
+        in, out, tab, g, status, groups, chunks);
+    return true;
+}
+
 template <typename T>
 int helical_run(int method, const ctr_helical_param* p, const T* in, T* out, const void* table, unsigned* status,
                 int batch, cudaStream_t stream)
@@ -534,10 +792,12 @@ int helical_run(int method, const ctr_helical_param* p, const T* in, T* out, con
         const float* fin = reinterpret_cast<const float*>(in);
         float* fout = reinterpret_cast<float*>(out);
         const dim3 grid(div_up(p->ns, kHeliThreads), div_up(p->view_per_rot, kHeliViews), p->nz * batch);
-        if (method == CTR_HELICAL_360)
+        if (method == CTR_HELICAL_360 && launch_360(p, g, fin, fout, tab, status, batch, stream)) {
+        } else if (method == CTR_HELICAL_360) {
             helical_fast_f32<CTR_HELICAL_360><<<grid, kHeliThreads, 0, stream>>>(fin, fout, tab, g, status);
-        else
+        } else {
             helical_fast_f32<CTR_HELICAL_180><<<grid, kHeliThreads, 0, stream>>>(fin, fout, tab, g, status);
+        }
         return check_launch(method == CTR_HELICAL_360 ? "helical 360LI (FP32)" : "helical 180LI (FP32)");
     }
     if (method == CTR_HELICAL_360)
