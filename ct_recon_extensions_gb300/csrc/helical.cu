@@ -488,6 +488,14 @@ __device__ __forceinline__ float ldg_above(const float* p, int n)
         : "l"(p), "r"(n), "n"(K));
     return v;
 }
+__device__ __forceinline__ float ldg_above_n(const float* p, int n, int k)
+{
+    float v;
+    asm("{\n\t.reg .pred q;\n\tsetp.gt.s32 q, %2, %3;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}"
+        : "=f"(v)
+        : "l"(p), "r"(n), "r"(k));
+    return v;
+}
 __device__ __forceinline__ float ldg_negative(const float* p, float x)
 {
     float v;
@@ -503,7 +511,7 @@ __device__ __forceinline__ float ldg_negative(const float* p, float x)
 struct H3Edge {
     float k, a;
     int all;
-    bool sure;
+    bool two, sure;  // the channels' edges lie on both sides of `all`; or not decided here
 };
 
 enum H3Kind { kH3None, kH3Rows, kH3Mixed, kH3Two, kH3Slow };
@@ -519,15 +527,16 @@ struct H3View {
 };
 static_assert(sizeof(H3View) == 32, "16-byte loads");
 
-__device__ __forceinline__ H3Edge h3_edge(const HeliGeo& g, float a, float g0, float g1, float guard, bool top)
+// An edge that lies in [lo, hi] over the channels, at k - a g past a lane's integer.
+__device__ __forceinline__ H3Edge h3_edge(const HeliGeo& g, float a, float lo, float hi, float guard, bool top)
 {
-    const float x0 = g.ct_f - a * g0, x1 = g.ct_f - a * g1;
-    const float lo = fminf(x0, x1), hi = fmaxf(x0, x1), fl = floorf(lo), fh = floorf(hi);
+    const float fl = floorf(lo), fh = floorf(hi);
     // all edges clamped to the detector's end: floor(max(x, 0)) = 0, ceil(min(x, nt)) = nt
     const bool clamped = top ? hi < 1.0f - guard : lo > g.nt_f - 1.0f + guard;
     H3Edge e;
     const bool away = lo - fl > guard && fh + 1.0f - hi > guard;
     const bool two = !clamped && fh == fl + 1.0f;
+    e.two = two;
     e.sure = clamped || (away && (fh == fl || two));
     const float row = top ? (clamped ? 0.0f : fh) : (clamped ? g.nt_f : (two ? fh : fl + 1.0f));
     e.all = static_cast<int>(row);
@@ -536,32 +545,38 @@ __device__ __forceinline__ H3Edge h3_edge(const HeliGeo& g, float a, float g0, f
     return e;
 }
 
-// The rows of one sample's slab with the quotients a (top) and b (bottom):
-// false where they are left to heli_fast_one; n = 0 and no edge where it misses.
-__device__ __forceinline__ bool h3_rows(const HeliGeo& g, float a, float b, float g0, float g1, float guard, H3Edge& t,
-                                        H3Edge& e)
+// The rows of one sample's slab with the quotients a (top) and b (bottom), x =
+// ct - a g less up to `more` over the channels' g in [g0, g1]: false where they
+// are left to heli_fast_one, no rows (t.all = 0, e.all = -1) where it misses for
+// all.  A lane's slab that misses where another's does not has no rows either:
+// its bottom edge lies below row 0 or its top edge past the last one.
+__device__ __forceinline__ bool h3_rows(const HeliGeo& g, float a, float b, float g0, float g1, float more, float guard,
+                                        H3Edge& t, H3Edge& e)
 {
-    t = e = H3Edge{0.0f, 0.0f, 0, true};
+    t = e = H3Edge{0.0f, 0.0f, 0, false, true};
     t.k = 1.0f;
     e.k = -1.0f;
-    const float b0 = g.ct_f - b * g0, b1 = g.ct_f - b * g1, t0 = g.ct_f - a * g0, t1 = g.ct_f - a * g1;
-    if (fmaxf(b0, b1) < -guard || fminf(t0, t1) >= g.nt_f + guard) return true;  // misses for every channel
-    if (fminf(b0, b1) <= guard || fmaxf(t0, t1) >= g.nt_f - guard) return false;
-    t = h3_edge(g, a, g0, g1, guard, true);
-    e = h3_edge(g, b, g0, g1, guard, false);
+    e.all = -1;
+    const float t0 = g.ct_f - a * g0, t1 = g.ct_f - a * g1, b0 = g.ct_f - b * g0, b1 = g.ct_f - b * g1;
+    const float up = fmaxf(more, 0.0f), down = fminf(more, 0.0f);
+    const float tl = fminf(t0, t1) - up, th = fmaxf(t0, t1) - down, bl = fminf(b0, b1) - up, bh = fmaxf(b0, b1) - down;
+    if (bh < -guard || tl >= g.nt_f + guard) return true;  // misses for every channel
+    t = h3_edge(g, a, tl, th, guard, true);
+    e = h3_edge(g, b, bl, bh, guard, false);
     return t.sure && e.sure && e.all >= t.all;
 }
 
 // A sample that its task left.  Out of line: its registers would halve the
 // kernel's blocks an SM.
+template <int M>
 __device__ __noinline__ void h3_slow(const float* in, float* out, const HeliHeader* tab, const HeliGeo& g,
                                      unsigned* status, unsigned iz, unsigned iv, unsigned is)
 {
-    const HeliSlice* slices = heli_slices<CTR_HELICAL_360>(tab, g);
+    const HeliSlice* slices = heli_slices<M>(tab, g);
     const HeliChanF cf = reinterpret_cast<const HeliChanF*>(slices + g.nz)[is];
     const size_t row = static_cast<size_t>(iz) * g.vpr + iv;
-    heli_fast_one<CTR_HELICAL_360>(in, out + row * g.ns + is, tab, g, slices[iz],
-                                   heli_rows_f<CTR_HELICAL_360>(tab, g)[row], cf, iv, is, status + iz);
+    heli_fast_one<M>(in, out + row * g.ns + is, tab, g, slices[iz],
+                                   heli_rows_f<M>(tab, g)[row], cf, iv, is, status + iz);
 }
 
 __global__ void __launch_bounds__(32 * kH3Warps, 12)
@@ -606,10 +621,10 @@ __global__ void __launch_bounds__(32 * kH3Warps, 12)
     if (valid && iv < g.vpr) {
         const HeliRowF& r = rows[static_cast<size_t>(iz) * g.vpr + iv];
         H3Edge t1, b1, t2, b2;
-        const bool sure = h3_rows(g, r.at, r.ab, g0, g1, guard, t1, b1) &&
-                          h3_rows(g, r.at2, r.ab2, g0, g1, guard, t2, b2);
-        const bool hit1 = b1.all > 0, hit2 = b2.all > 0;  // the last row's end
-        const bool mixed = t1.a != 0.0f || b1.a != 0.0f || t2.a != 0.0f || b2.a != 0.0f;
+        const bool sure = h3_rows(g, r.at, r.ab, g0, g1, 0.0f, guard, t1, b1) &&
+                          h3_rows(g, r.at2, r.ab2, g0, g1, 0.0f, guard, t2, b2);
+        const bool hit1 = b1.all >= 0, hit2 = b2.all >= 0;
+        const bool mixed = t1.two || b1.two || t2.two || b2.two;
         kind = !sure || !(hit1 || hit2) ? kH3Slow : hit1 && hit2 ? kH3Two : mixed ? kH3Mixed : kH3Rows;
         auto view = [&](int i, int from, const H3Edge& top, const H3Edge& bot, float w) {
             H3View v;
@@ -647,14 +662,14 @@ __global__ void __launch_bounds__(32 * kH3Warps, 12)
         for (int r = 4; r < n; ++r) s += __ldg(in + (at + r * ns));
         return s;
     };
-    // the mean of a lane's rows; near: a lane's edge is too close to the integer
-    auto mean = [&](const H3View& v, bool& near) {
+    // the mean of a lane's rows, of which it may have none; near: a lane's edge
+    // is too close to the integer
+    auto mean = [&](const H3View& v, int& n, bool& near) {
         const float dt = fmaf(-v.ta, gc, v.tk), db = fmaf(v.ba, gc, -v.bk);  // minus what b lies past its integer
         near = near || fminf(fabsf(dt), fabsf(db)) < guard;
         const unsigned at = v.at + is;
-        int n = v.n;
-        const float s = (ldg_negative(in + (at - ns), dt) + ldg_negative(in + (at + n * ns), db)) + sum(at, n);
-        n += (dt < 0.0f ? 1 : 0) + (db < 0.0f ? 1 : 0);
+        const float s = (ldg_negative(in + (at - ns), dt) + ldg_negative(in + (at + v.n * ns), db)) + sum(at, v.n);
+        n = v.n + (dt < 0.0f ? 1 : 0) + (db < 0.0f ? 1 : 0);
         return __fdividef(s, static_cast<float>(n));
     };
     while (m_rows) {
@@ -679,8 +694,10 @@ __global__ void __launch_bounds__(32 * kH3Warps, 12)
         bool near[kH3Group];
 #pragma unroll
         for (int u = 0; u < kH3Group; ++u) {
+            int n;
             near[u] = false;
-            v[u] = mean(s_view[0][warp][k[u]], near[u]);
+            v[u] = mean(s_view[0][warp][k[u]], n, near[u]);
+            near[u] = near[u] || n < 1;  // no row at all
         }
 #pragma unroll
         for (int u = 0; u < kH3Group; ++u) {
@@ -692,14 +709,236 @@ __global__ void __launch_bounds__(32 * kH3Warps, 12)
         const int k = __ffs(m_two) - 1;
         bool near = false;
         const H3View a = s_view[0][warp][k], c = s_view[1][warp][k];
-        const float ma = mean(a, near), mc = mean(c, near);
-        if (__any_sync(0xffffffffu, near)) slow |= 1u << k;
-        else if (on) out[a.out + is] = fmaf(c.w, mc, a.w * ma);
+        int na, nc;
+        const float ma = mean(a, na, near), mc = mean(c, nc, near);
+        if (__any_sync(0xffffffffu, near || na + nc < 1)) slow |= 1u << k;
+        else if (on) out[a.out + is] = na < 1 ? mc : nc < 1 ? ma : fmaf(c.w, mc, a.w * ma);
     }
     for (; slow && on; slow &= slow - 1) {  // sample by sample
         const int k = __ffs(slow) - 1;
-        h3_slow(in, out, tab, g, status, iz0 + k % kH3Slices, blockIdx.y * kH3Views + k / kH3Slices, is);
+        h3_slow<CTR_HELICAL_360>(in, out, tab, g, status, iz0 + k % kH3Slices, blockIdx.y * kH3Views + k / kH3Slices, is);
     }
+}
+
+// ---- 180LI, FP32: complementary rays along their views --------------------------
+// The complementary ray of output view `cur` and channel is lies dif(is) views
+// back, between views k - 1 and k = cur - floor(dif), wrapped into the slice's
+// views, at the mirrored channel.  dif changes by half a view from channel to
+// channel, so the rays of 32 channels at one output view lie in ~14 views, and
+// every load touches as many rows.  A warp takes 32 channels (one a lane) of
+// kH8Views output views of a slice instead in three steps: the measured samples,
+// output view by output view, into shared memory; the complementary ones, view k
+// by view k (a lane's output view is k + floor(dif), idle where that is not of
+// the group), where the lanes' channels are adjacent and the sum over view k's
+// rows is the next step's sum over view k - 1 while the rows stay the same; then
+// the interpolated rows out.  Detector rows are decided as in helical_360_f32;
+// a lane's complementary edges also depend on its fraction of dif.  A view's
+// rows are kept as a window of NR registers a lane, of which it sums its own.
+// Issue bound: 128 slices x 1152 views x 736 channels 1815 -> 1221 us.  With each
+// lane's sums formed from memory instead of a window 1523 us, a branch per row
+// count 1280 us, 64 views a warp 1660 us, 10 blocks an SM spilled.
+constexpr int kH8Views = 32, kH8Warps = 4;
+static_assert(kH8Views == 32, "a view a lane, a lane's views in a 32-bit mask");
+
+template <int NR>
+__global__ void __launch_bounds__(32 * kH8Warps, 8)
+    helical_180_f32(const float* __restrict__ in, float* __restrict__ out, const HeliHeader* __restrict__ tab,
+                    const __grid_constant__ HeliGeo g, unsigned* status, unsigned chunks)
+{
+    extern __shared__ __align__(16) float s_dyn[];  // per warp: values [view][lane], 32 tasks, z distances
+    constexpr int kWarpFloats = kH8Views * 32 + 32 * 8 + kH8Views;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float* s_val = s_dyn + warp * kWarpFloats;
+    H3View* s_task = reinterpret_cast<H3View*>(s_val + kH8Views * 32);
+    float* s_zd = s_val + kH8Views * 32 + 32 * 8;
+    const unsigned b = blockIdx.z / g.nz, iz = blockIdx.z - b * g.nz;
+    const unsigned chunk = blockIdx.x * kH8Warps + warp, c0 = chunk * 32;
+    if (chunk >= chunks) return;  // warp-uniform
+    const HeliSlice s = heli_slices<CTR_HELICAL_180>(tab, g)[iz];
+    if (!heli_slice_ok<CTR_HELICAL_180>(tab, g, s, status)) return;
+    in += b * g.in_item;
+    out += b * g.out_item;
+    status += b * g.nz;
+    const bool on = c0 + lane < g.ns;
+    const unsigned is = min(c0 + lane, g.ns - 1), ns = g.ns;
+    const unsigned iv0 = blockIdx.y * kH8Views;
+    const int nv = min(static_cast<int>(g.vpr - iv0), kH8Views), vpr = static_cast<int>(g.vpr);
+    const HeliChanF cf = reinterpret_cast<const HeliChanF*>(heli_slices<CTR_HELICAL_180>(tab, g) + g.nz)[is];
+    const HeliRowF* rows = heli_rows_f<CTR_HELICAL_180>(tab, g) + static_cast<size_t>(iz) * g.vpr;
+    const float cm = g.vprcm_f / static_cast<float>(vpr);  // couch travel of a view
+    float g0 = cf.g, g1 = cf.g, h0 = cf.h, h1 = cf.h;
+    int d0 = cf.dif_i, d1 = cf.dif_i;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        g0 = fminf(g0, __shfl_xor_sync(0xffffffffu, g0, o));
+        g1 = fmaxf(g1, __shfl_xor_sync(0xffffffffu, g1, o));
+        h0 = fminf(h0, __shfl_xor_sync(0xffffffffu, h0, o));
+        h1 = fmaxf(h1, __shfl_xor_sync(0xffffffffu, h1, o));
+        d0 = min(d0, __shfl_xor_sync(0xffffffffu, d0, o));
+        d1 = max(d1, __shfl_xor_sync(0xffffffffu, d1, o));
+    }
+    const float guard = kEdgeGuard + (g.nt_f + 1.0f + fabsf(g.ct_f)) * kEdgeGuardRel;
+    unsigned left = on && cf.exact ? ~0u : 0u;  // this lane's samples left to h3_slow
+    unsigned has = 0;                           // its views whose measured slab meets the detector
+
+    // a task: the edges' rows over the channels, or -1 (misses) or -2 (left) in n
+    auto decide = [&](float a, float bq, float q0, float q1, float more, int view, H3View& t) {
+        H3Edge te, be;
+        const bool sure = h3_rows(g, a, bq, q0, q1, more, guard, te, be);
+        t.n = !sure ? -2 : be.all - te.all;
+        t.at = (static_cast<unsigned>(view) * g.nt + te.all) * ns;
+        t.tk = te.k;
+        t.ta = te.a;
+        t.bk = be.k;
+        t.ba = be.a;
+        t.out = (te.two ? 1u : 0u) | (be.two ? 2u : 0u);  // lanes differ
+    };
+    // rows of a lane: whether it has the one above the common ones and the one below
+    auto extra = [&](const H3View& t, float gc, float off, bool& above, bool& below) {
+        const float dt = fmaf(-t.ta, gc, t.tk - off), db = fmaf(-t.ba, gc, t.bk - off);
+        above = dt < 0.0f;
+        below = db >= 0.0f;
+        return fminf(fabsf(dt), fabsf(db)) < guard;
+    };
+
+    // 1. the measured samples
+    {
+        if (lane < nv) {
+            const HeliRowF& r = rows[iv0 + lane];
+            H3View t;
+            decide(r.at, r.ab, g0, g1, 0.0f, r.cur, t);
+            t.w = t.n > 0 ? __fdividef(1.0f, static_cast<float>(t.n)) : 0.0f;
+            s_task[lane] = t;
+            s_zd[lane] = r.zd;
+        }
+        __syncwarp();
+        for (int v = 0; v < nv; ++v) {
+            const H3View t = s_task[v];
+            if (t.n == -2) {
+                left |= 1u << v;
+                continue;
+            }
+            if (t.n == -1) continue;
+            bool any = true;
+            const unsigned at = t.at + is;
+            float m = (ldg_above<0>(in + at, t.n) + ldg_above<1>(in + (at + ns), t.n)) +
+                      (ldg_above<2>(in + (at + 2 * ns), t.n) + ldg_above<3>(in + (at + 3 * ns), t.n));
+            for (int r = 4; r < t.n; ++r) m += __ldg(in + (at + r * ns));
+            if (t.out) {
+                bool above, below;
+                if (extra(t, cf.g, 0.0f, above, below)) left |= 1u << v;
+                m += ldg_above<0>(in + (at - ns), above) + ldg_above<0>(in + (at + t.n * ns), below);
+                any = t.n + above + below > 0;
+                m = __fdividef(m, static_cast<float>(t.n + above + below));
+            } else {
+                m *= t.w;
+            }
+            has |= any ? 1u << v : 0u;
+            s_val[v * 32 + lane] = m;
+        }
+        __syncwarp();
+    }
+
+    // 2. the complementary samples: K runs over the unwrapped views cur - floor(dif)
+    const int base = s.first + static_cast<int>(iv0);
+    const float f = 1.0f - cf.u, off = f * cm * cf.h;  // the fraction of dif, and its way along the rows
+    const unsigned cl = max(cf.cl, 0), cr = max(cf.cr, 0);
+    const float w = 1.0f - cf.v;
+    const int k0 = base - d1, k1 = base + nv - 1 - d0;
+    const unsigned view = g.nt * ns;
+    float right[NR], leftv[NR];  // the window's rows of views k and k - 1 at the lane's mirrored channel
+    unsigned held = 0;  // the element that `right` starts at, and its rows
+    int held_n = 0;
+    for (int kb = k0; kb <= k1; kb += 32) {
+        if (kb + lane <= k1) {
+            int k = kb + lane;
+            k += k < s.lo ? vpr : (k > s.hi ? -vpr : 0);
+            const int ivk = k - s.first + (k < s.first ? vpr : 0);
+            const float zd = rows[ivk].zd;
+            H3View t;
+            decide(zd + g.hth_f, zd - g.hth_f, h0, h1, cm * h1, k, t);
+            // the window: the common rows and, where lanes differ at an edge (k away from 1 and -1), the one beyond
+            const unsigned above = t.out & 1u, below = t.out >> 1;
+            if (t.n >= 0) {
+                t.at -= above * ns;
+                t.n += above + below;
+                if (t.n > NR) t.n = -2;
+            }
+            if (k == 0) t.n = -2;  // view k - 1 lies before the scan
+            t.w = zd;
+            s_task[lane] = t;
+        }
+        __syncwarp();
+        for (int j = 0; j < min(32, k1 - kb + 1); ++j) {
+            const H3View t = s_task[j];
+            const int v = kb + j + cf.dif_i - base;
+            const bool act = static_cast<unsigned>(v) < static_cast<unsigned>(nv);
+            const unsigned bit = act ? 1u << v : 0u;
+            if (t.n < 1) {
+                held_n = 0;
+                // no complementary row: the measured sample as it is, where there is one
+                left |= t.n == -2 ? bit : bit & ~has;
+                continue;
+            }
+            auto window = [&](float (&c)[NR], unsigned at) {
+                const float* p = in + (at + cl);
+                const float* q = in + (at + cr);
+#pragma unroll
+                for (int r = 0; r < NR; ++r)  // 0 past the window
+                    c[r] = fmaf(w, ldg_above_n(p + r * ns, t.n, r), cf.v * ldg_above_n(q + r * ns, t.n, r));
+            };
+            if (held_n >= t.n && held == t.at - view) {
+#pragma unroll
+                for (int r = 0; r < NR; ++r) leftv[r] = right[r];
+            } else {
+                window(leftv, t.at - view);
+            }
+            window(right, t.at);
+            held = t.at;
+            held_n = t.n;
+            int n = t.n;
+            float sl = leftv[0], sr = right[0];
+            if (t.out) {  // the lane's rows of the window
+                const float dt = fmaf(-t.ta, cf.h, t.tk - off), db = fmaf(-t.ba, cf.h, t.bk - off);
+                if (fminf(fabsf(dt), fabsf(db)) < guard) left |= bit;
+                const int from = (t.out & 1u) && dt >= 0.0f ? 1 : 0, to = t.n - ((t.out & 2u) && db < 0.0f ? 1 : 0);
+                n = to - from;
+                if (from > 0 || n < 1) sl = sr = 0.0f;
+#pragma unroll
+                for (int r = 1; r < NR; ++r)
+                    if (r < to) {
+                        sl += leftv[r];
+                        sr += right[r];
+                    }
+            } else {
+#pragma unroll
+                for (int r = 1; r < NR; ++r) {
+                    sl += leftv[r];
+                    sr += right[r];
+                }
+            }
+            if (n < 1) left |= bit & ~has;
+            if (!act || n < 1) continue;
+            const float vcor = __fdividef(fmaf(f, sl, cf.u * sr), static_cast<float>(n));
+            const float zd = s_zd[v], zd2 = t.w + f * cm;
+            float val = vcor;
+            if (cf.cl < 0) {  // mirrored channel off the detector: no interpolation
+                val = has & bit ? s_val[v * 32 + lane] : 0.0f;
+            } else if (has & bit) {
+                val = __fdividef(zd * vcor - zd2 * s_val[v * 32 + lane], zd - zd2);
+            }
+            s_val[v * 32 + lane] = val;
+        }
+        __syncwarp();
+    }
+
+    // 3. out
+    const unsigned to = (iz * g.vpr + iv0) * ns + is;
+    for (int v = 0; v < nv; ++v)
+        if (on && !(left >> v & 1)) out[to + v * ns] = s_val[v * 32 + lane];
+    // each lane its own next sample: the lanes' views differ
+    for (left = on ? left & (~0u >> (32 - nv)) : 0u; left; left &= left - 1)
+        h3_slow<CTR_HELICAL_180>(in, out, tab, g, status, iz, iv0 + __ffs(left) - 1, is);
 }
 
 size_t table_bytes(const ctr_helical_param* p)
@@ -774,6 +1013,37 @@ bool launch_360(const ctr_helical_param* p, const HeliGeo& g, const float* in, f
     return true;
 }
 
+// 180LI view by view: false (nothing launched) where an item's elements need
+// more than 32 bits, a complementary ray lies a rotation or more away, or the
+// slab covers more rows than the window, and for small scans.
+bool launch_180(const ctr_helical_param* p, const HeliGeo& g, const float* in, float* out, const HeliHeader* tab,
+                unsigned* status, int batch, cudaStream_t stream)
+{
+    const double center_s = static_cast<double>(p->ns - 1) / 2.0 + p->offset_s;
+    for (double c : {0.0, static_cast<double>(p->ns - 1)}) {
+        const double dif = (kHeliPi - 2 * (c - center_s) * p->ds / p->dsd) / p->orbit;
+        if (!(dif >= 0.0 && dif <= static_cast<double>(p->view_per_rot) - 1.0)) return false;
+    }
+    if (g.in_item > 0xffffffffu || g.out_item > 0xffffffffu) return false;
+    const unsigned chunks = div_up(p->ns, 32);
+    constexpr size_t smem = sizeof(float) * kH8Warps * (kH8Views * 32 + 32 * 8 + kH8Views);
+    const unsigned views = div_up(p->view_per_rot, kH8Views);
+    const dim3 grid(div_up(chunks, kH8Warps), views, p->nz * batch);
+    // Few warps leave the steps' latency bare: 960 warps (8 slices x 360 views x
+    // 300 channels) 39 us against 31 sample by sample, 3840 warps (16 x 500 x
+    // 450) 58 against 83.  An item's count, so that an item's values are the same
+    // in any batch.
+    if (static_cast<size_t>(chunks) * views * p->nz < 2048) return false;
+    const double slab = p->thickness * p->dsd / p->dso;  // in rows, at the centre channel
+    if (slab <= 2.5)
+        helical_180_f32<4><<<grid, 32 * kH8Warps, smem, stream>>>(in, out, tab, g, status, chunks);
+    else if (slab <= 6.0)
+        helical_180_f32<8><<<grid, 32 * kH8Warps, smem, stream>>>(in, out, tab, g, status, chunks);
+    else
+        return false;
+    return true;
+}
+
 template <typename T>
 int helical_run(int method, const ctr_helical_param* p, const T* in, T* out, const void* table, unsigned* status,
                 int batch, cudaStream_t stream)
@@ -792,12 +1062,12 @@ int helical_run(int method, const ctr_helical_param* p, const T* in, T* out, con
         const float* fin = reinterpret_cast<const float*>(in);
         float* fout = reinterpret_cast<float*>(out);
         const dim3 grid(div_up(p->ns, kHeliThreads), div_up(p->view_per_rot, kHeliViews), p->nz * batch);
-        if (method == CTR_HELICAL_360 && launch_360(p, g, fin, fout, tab, status, batch, stream)) {
-        } else if (method == CTR_HELICAL_360) {
+        const bool done = method == CTR_HELICAL_360 ? launch_360(p, g, fin, fout, tab, status, batch, stream)
+                                                    : launch_180(p, g, fin, fout, tab, status, batch, stream);
+        if (!done && method == CTR_HELICAL_360)
             helical_fast_f32<CTR_HELICAL_360><<<grid, kHeliThreads, 0, stream>>>(fin, fout, tab, g, status);
-        } else {
+        else if (!done)
             helical_fast_f32<CTR_HELICAL_180><<<grid, kHeliThreads, 0, stream>>>(fin, fout, tab, g, status);
-        }
         return check_launch(method == CTR_HELICAL_360 ? "helical 360LI (FP32)" : "helical 180LI (FP32)");
     }
     if (method == CTR_HELICAL_360)

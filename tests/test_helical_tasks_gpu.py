@@ -15,7 +15,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("method", ["360", "180"])
 @pytest.mark.parametrize("ns,nt,vpr,nz,pitch,thickness", [
     (31, 8, 37, 3, 1.0, 0.3), (32, 16, 64, 8, 1.0, 1.0), (33, 16, 66, 9, 0.6, 2.0), (127, 32, 131, 17, 0.9, 6.0),
-    (129, 12, 200, 5, 1.0, 0.0), (200, 64, 97, 20, 0.45, 1.25)])
+    (129, 12, 200, 5, 1.0, 0.0), (200, 64, 97, 20, 0.45, 1.25),
+    (290, 16, 330, 20, 1.0, 1.0), (321, 20, 257, 23, 0.8, 2.5), (257, 16, 300, 24, 0.9, 0.0)])
 def test_helical_groups(port, method, ns, nt, vpr, nz, pitch, thickness):
     from oracle import Heli
     from ct_recon_extensions_gb300 import torch_ctrecon as tc
