@@ -194,4 +194,6 @@ def check(status: int, where: str) -> None:
 
 def call(name: str, *args) -> None:
     """Call an entry point and raise CtrError on a nonzero status."""
-    check(getattr(load(), name)(*args), name)
+    status = getattr(_lib or load(), name)(*args)
+    if status:
+        check(status, name)

@@ -30,12 +30,14 @@ _FILTER_TYPES = {"par": 0, "fan": 1, "flat": 2}
 _WEIGHT_TYPES = {"fan": 1, "flat": 2}
 
 
-def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream() -> int:
+    """The current stream's handle.  Read without building a Stream object: 0.1
+    us against 3.1 of torch.cuda.current_stream(), on every call."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def _ptr(t: torch.Tensor):
-    return ctypes.c_void_p(t.data_ptr())
+def _ptr(t: torch.Tensor) -> int:
+    return t.data_ptr()  # the entry points' void* arguments take an int
 
 
 def _sfx(t: torch.Tensor) -> str:
