@@ -1369,42 +1369,43 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// The 4n - 4 border pixels, exactly, overwriting fp_adj_f32's values: one
-// 128-thread block per pixel and up to kFbImg images (blockIdx.y*kFbImg ..).
-// Thread t sums views t, t+128, ... of each image (the taps of a view are
-// planned once for all images), then a fixed tree: a shuffle tree per warp,
-// the four warps in order.
-constexpr int kFbImg = 8;
-__global__ void __launch_bounds__(128)
+// The 4n - 4 border pixels, exactly, overwriting fp_adj_f32's values: a block
+// takes kFbPix adjacent pixels of one edge and up to IMG images (blockIdx.y *
+// IMG ..), thread (pixel, q) sums views q, q + kFbViews, ... of each image
+// (the taps of a view are planned once for all images), then a fixed tree over
+// the kFbViews sums.  Adjacent pixels read adjacent positions and channels: with
+// one pixel a block and a view a lane each load touched 32 sectors (512^2, 720
+// views: 19 us for one image and 116 for 16, now 10 and 52).  64 views at a
+// time: the loop is a chain of three dependent loads (32: 16 us for one image).
+constexpr int kFbImg = 4;
+constexpr int kFbPix = 8;
+constexpr int kFbViews = 64;
+template <int IMG>
+__global__ void __launch_bounds__(kFbPix * kFbViews, 2)
     fp_adj_border_f32(const float* __restrict__ proj, float* __restrict__ img,
                       const long long* __restrict__ B, const AdjView* __restrict__ V,
                       const double* __restrict__ pos, const FpConst c, int batch)
 {
-    __shared__ float s_part[4][kFbImg];
+    __shared__ float s_part[IMG][kFbViews / 4][kFbPix];
     const int n = c.nx, ns = c.ns;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int b = blockIdx.x;
-    int ix, iy;
-    if (b < n) {
-        ix = b;
-        iy = 0;
-    } else if (b < 2 * n) {
-        ix = b - n;
-        iy = n - 1;
-    } else if (b < 3 * n - 2) {
-        ix = 0;
-        iy = b - 2 * n + 1;
-    } else {
-        ix = n - 1;
-        iy = b - 3 * n + 3;
-    }
-    const int im0 = blockIdx.y * kFbImg;
-    const int cnt = min(kFbImg, batch - im0);
+    const int k = threadIdx.x % kFbPix, q = threadIdx.x / kFbPix;
+    // edges: the first and last row, the first and last column (without its
+    // corners), in whole blocks
+    const int per = (n + kFbPix - 1) / kFbPix;
+    const int edge = blockIdx.x / per;
+    const int at = (blockIdx.x - edge * per) * kFbPix + k;
+    const bool live = edge < 2 ? at < n : at > 0 && at < n - 1;
+    const int p = min(at, n - 1);
+    const int ix = edge < 2 ? p : (edge == 2 ? 0 : n - 1);
+    const int iy = edge < 2 ? (edge == 0 ? 0 : n - 1) : p;
+    const int im0 = blockIdx.y * IMG;
+    const int cnt = min(IMG, batch - im0);
     const float* P = proj + static_cast<size_t>(im0) * c.proj_stride;
-    float acc[kFbImg];
+    float acc[IMG];
 #pragma unroll
-    for (int i = 0; i < kFbImg; ++i) acc[i] = 0.0f;
-    for (int ia = threadIdx.x; ia < c.na; ia += 128) {
+    for (int i = 0; i < IMG; ++i) acc[i] = 0.0f;
+#pragma unroll 1
+    for (int ia = q; ia < c.na; ia += kFbViews) {
         const AdjView v = V[ia];
         const int along = v.ux ? ix : iy, lin = v.ux ? iy : ix;
         const size_t line = static_cast<size_t>(ia) * n + lin;
@@ -1414,32 +1415,39 @@ __global__ void __launch_bounds__(128)
         if (t.two) {  // every image's two loads issued before the first FMA
             const bool in0 = static_cast<unsigned>(t.mi) < static_cast<unsigned>(ns);
             const bool in1 = static_cast<unsigned>(t.mi + 1) < static_cast<unsigned>(ns);
-            float p0[kFbImg], p1[kFbImg];
+            float p0[IMG], p1[IMG];
 #pragma unroll
-            for (int i = 0; i < kFbImg; ++i) {
+            for (int i = 0; i < IMG; ++i) {
                 const float* r = row + i * c.proj_stride;
                 p0[i] = i < cnt && in0 ? __ldg(r + t.mi) : 0.0f;
                 p1[i] = i < cnt && in1 ? __ldg(r + t.mi + 1) : 0.0f;
             }
 #pragma unroll
-            for (int i = 0; i < kFbImg; ++i) acc[i] = fmaf(fmaf(t.w0, p0[i], t.w1 * p1[i]), v.w, acc[i]);
+            for (int i = 0; i < IMG; ++i) acc[i] = fmaf(fmaf(t.w0, p0[i], t.w1 * p1[i]), v.w, acc[i]);
         } else {
 #pragma unroll
-            for (int i = 0; i < kFbImg; ++i)
+            for (int i = 0; i < IMG; ++i)
                 if (i < cnt) acc[i] = fmaf(adj_tap_apply(row + i * c.proj_stride, t, v.inv, ns), v.w, acc[i]);
         }
     }
+    // a warp holds 4 views' sums of each pixel
 #pragma unroll
-    for (int i = 0; i < kFbImg; ++i) {
+    for (int i = 0; i < IMG; ++i) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
-        if (lane == 0) s_part[warp][i] = acc[i];
+        for (int o = kFbPix; o < 32; o <<= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+        if ((q & 3) == 0) s_part[i][q >> 2][k] = acc[i];
     }
     __syncthreads();
-    if (threadIdx.x < cnt) {
-        const int i = threadIdx.x;
-        const float sum = ((s_part[0][i] + s_part[1][i]) + s_part[2][i]) + s_part[3][i];
-        img[static_cast<size_t>(im0 + i) * c.img_stride + static_cast<size_t>(iy) * n + ix] = sum;
+    if (q < cnt && live) {
+        float s[kFbViews / 4];
+#pragma unroll
+        for (int w = 0; w < kFbViews / 4; ++w) s[w] = s_part[q][w][k];
+#pragma unroll
+        for (int o = 1; o < kFbViews / 4; o <<= 1)
+#pragma unroll
+            for (int w = 0; w < kFbViews / 4; w += 2 * o) s[w] += s[w + o];
+        const float sum = s[0];
+        img[static_cast<size_t>(im0 + q) * c.img_stride + static_cast<size_t>(iy) * n + ix] = sum;
     }
 }
 
@@ -1857,9 +1865,13 @@ int fp_adjoint(const ctr_par_param* p, const T* proj, T* img, const double* w,
                 std::min<size_t>(div_up(vec ? count / 4 : count, 256), 8ull * sms));
             fp_adj_reduce<<<blocks, 256, 0, stream>>>(part, img, count, segs, vec);
         }
-        const unsigned nborder = p->nx == 1 ? 1u : 4u * p->nx - 4u;
-        fp_adj_border_f32<<<dim3(nborder, div_up(batch, kFbImg)), 128, 0, stream>>>(proj, img, B, V, pos, c,
-                                                                                  batch);
+        const unsigned edges = p->nx == 1 ? 1u : 4u;
+        const unsigned blocks = edges * static_cast<unsigned>(div_up(p->nx, kFbPix));
+        if (batch == 1)
+            fp_adj_border_f32<1><<<blocks, kFbPix * kFbViews, 0, stream>>>(proj, img, B, V, pos, c, batch);
+        else
+            fp_adj_border_f32<kFbImg><<<dim3(blocks, div_up(batch, kFbImg)), kFbPix * kFbViews, 0, stream>>>(
+                proj, img, B, V, pos, c, batch);
         cudaFreeAsync(scratch, stream);  // after every kernel that reads the tables
     } else {
         dim3 grid(div_up(p->nx, 32), div_up(p->ny, 8), batch);
