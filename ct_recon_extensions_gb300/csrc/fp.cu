@@ -962,9 +962,10 @@ __global__ void __launch_bounds__(kFpxThreads, 1)
 // images, and two FMAs per image; positions advance by 64-bit adds.  It
 // computes every pixel that way.  Pixels on the image border have one-sided
 // footprints (channels on the neighbour's side only); fp_adj_border_f32 then
-// recomputes those 4n - 4 pixels exactly and overwrites them.  When one image's
-// tiles would not fill the GPU, each tile's views are split into segments whose
-// partial images fp_adj_reduce sums in segment order.
+// recomputes those 4n - 4 pixels exactly and overwrites them.  Each tile's views
+// are split into segments, summed in segment order: by launches that add to the
+// image one after another, or, where the tiles would not fill the GPU, from
+// partial images by fp_adj_reduce.
 // Views with |offset| > 1 or a window wider than the staged one take the exact
 // per-pixel path in both kernels.
 constexpr int kFaViews = 16;
@@ -1182,9 +1183,12 @@ __device__ __forceinline__ void adj_tap_staged(float (&blk)[IMG][ROWS], int r, l
 }
 
 // The gather: CTA = one 32 x 8*ROWS tile of IMG images and one segment of
-// seg_len views: blockIdx.z = group * segs + segment, images img0 + group*IMG ...
-// With one segment it writes the images; with several, segment s writes its
-// partial sums to part[s][image] for fp_adj_reduce.  Per block of kFaViews views: one phase loads the tile's line positions and
+// seg_len views: blockIdx.z = group * split + k for segment seg0 + k, images img0 +
+// group*IMG ...  With split == 1 it writes the images (seg0 == 0) or adds to them
+// what the launches of the segments before it have written; with several, segment
+// s writes its partial sums to part[s][image] for fp_adj_reduce.  A launch that
+// adds may start while the one before it ends (its CTAs fill the SMs that run
+// dry); it waits for that one where it first reads the images.  Per block of kFaViews views: one phase loads the tile's line positions and
 // the windows' pairs (all loads in flight), one barrier, compute, one barrier;
 // the next block's view constants and windows are copied (cp.async) during
 // the compute into the other half of s_v / s_w.
@@ -1192,7 +1196,7 @@ template <int ROWS, int IMG>
 __global__ void __launch_bounds__(256, ROWS * IMG >= 32 ? 2 : 3)
     fp_adj_f32(const float* __restrict__ proj, float* __restrict__ img, const long long* __restrict__ B,
                const AdjView* __restrict__ V, const AdjWin* __restrict__ W, const double* __restrict__ pos,
-               const FpConst c, int img0, int segs, int seg_len, float* __restrict__ part, int batch)
+               const FpConst c, int img0, int split, int seg0, int seg_len, float* __restrict__ part, int batch)
 {
     using S = FaShape<ROWS>;
     constexpr int TY = S::TY, LINES = S::LINES, WIN = S::WIN;
@@ -1204,10 +1208,11 @@ __global__ void __launch_bounds__(256, ROWS * IMG >= 32 ? 2 : 3)
     float(*s_pair)[WIN][2 * IMG] = reinterpret_cast<float(*)[WIN][2 * IMG]>(s_pair_dyn);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int tx0 = blockIdx.x * kFaTileX, ty0 = blockIdx.y * TY;
     const int ix = tx0 + lane;
     const int ntiles = gridDim.x * gridDim.y, tile = blockIdx.y * gridDim.x + blockIdx.x;
-    const int seg = blockIdx.z % segs, im = img0 + (blockIdx.z / segs) * IMG;
+    const int seg = seg0 + blockIdx.z % split, im = img0 + (blockIdx.z / split) * IMG;
     const int vb = seg * seg_len, ve = min(c.na, vb + seg_len);
     const float* P = proj + static_cast<size_t>(im) * c.proj_stride;
     const int n = c.nx;  // == ny
@@ -1327,14 +1332,19 @@ __global__ void __launch_bounds__(256, ROWS * IMG >= 32 ? 2 : 3)
         cp_async_wait_all();
         __syncthreads();
     }
+    const bool add = split == 1 && seg0 > 0;
+    if (add) asm volatile("griddepcontrol.wait;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < IMG; ++i) {
-        float* O = segs == 1 ? img + static_cast<size_t>(im + i) * c.img_stride
-                             : part + (static_cast<size_t>(seg) * batch + im + i) * c.img_stride;
+        float* O = split == 1 ? img + static_cast<size_t>(im + i) * c.img_stride
+                              : part + (static_cast<size_t>(seg) * batch + im + i) * c.img_stride;
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
             const int iy = ty0 + warp * ROWS + r;
-            if (ix < c.nx && iy < c.ny) O[static_cast<size_t>(iy) * c.nx + ix] = acc[i][r];
+            if (ix < c.nx && iy < c.ny) {
+                float* o = O + static_cast<size_t>(iy) * c.nx + ix;
+                *o = add ? *o + acc[i][r] : acc[i][r];
+            }
         }
     }
 }
@@ -1794,25 +1804,42 @@ int fp_forward(const ctr_par_param* p, const T* img, T* proj, const double* sc,
 
 // The gather over a batch: CTAs of IMG images, the batch's remainder one image per CTA.
 template <int ROWS, int IMG>
-void fp_adj_launch(const float* proj, float* img, const long long* B, const AdjView* V, const AdjWin* W,
-                   const double* pos, const FpConst& c, int tiles_x, int tiles_y, int batch, int segs,
-                   int seg_len, float* part, cudaStream_t stream)
+cudaError_t fp_adj_launch(const float* proj, float* img, const long long* B, const AdjView* V, const AdjWin* W,
+                          const double* pos, const FpConst& c, int tiles_x, int tiles_y, int batch, int segs,
+                          int seg_len, float* part, cudaStream_t stream)
 {
     constexpr size_t smem = sizeof(float) * kFaViews * FaShape<ROWS>::WIN * 2 * IMG;
     constexpr size_t smem1 = sizeof(float) * kFaViews * FaShape<ROWS>::WIN * 2;
     if (smem > 48 * 1024)  // above the default limit (set per call: the current device's)
         cudaFuncSetAttribute(fp_adj_f32<ROWS, IMG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(smem));
-    const int groups = batch / IMG, zmax = 65535 / segs;  // grid z = groups x segments
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cfg.attrs = &early;
+    cudaError_t e = cudaSuccess;
+    // `count` CTAs' images from img0 on: every segment in one launch (part), or a
+    // launch a segment, each but the first adding to the one before it
+    auto launch = [&](auto kern, size_t bytes, int img0, int count) {
+        const int split = part ? segs : 1;
+        cfg.dynamicSmemBytes = bytes;
+        cfg.gridDim = dim3(tiles_x, tiles_y, count * split);
+        for (int seg = 0; seg < segs && e == cudaSuccess; seg += split) {
+            cfg.numAttrs = seg > 0 ? 1 : 0;
+            e = cudaLaunchKernelEx(&cfg, kern, proj, img, B, V, W, pos, c, img0, split, seg, seg_len, part, batch);
+        }
+    };
+    const int groups = batch / IMG, zmax = 65535 / segs;
     for (int g0 = 0; g0 < groups; g0 += zmax)
-        fp_adj_f32<ROWS, IMG><<<dim3(tiles_x, tiles_y, std::min(zmax, groups - g0) * segs), 256, smem, stream>>>(
-            proj, img, B, V, W, pos, c, g0 * IMG, segs, seg_len, part, batch);
+        launch(fp_adj_f32<ROWS, IMG>, smem, g0 * IMG, std::min(zmax, groups - g0));
     if constexpr (IMG > 1) {
         const int rest = batch - groups * IMG;
-        if (rest > 0)
-            fp_adj_f32<ROWS, 1><<<dim3(tiles_x, tiles_y, rest * segs), 256, smem1, stream>>>(
-                proj, img, B, V, W, pos, c, groups * IMG, segs, seg_len, part, batch);
+        if (rest > 0) launch(fp_adj_f32<ROWS, 1>, smem1, groups * IMG, rest);
     }
+    return e;
 }
 
 template <typename T>
@@ -1829,13 +1856,18 @@ int fp_adjoint(const ctr_par_param* p, const T* proj, T* img, const double* w,
         const int ty = FaShape<kRows>::TY, win = FaShape<kRows>::WIN;
         const int tiles_x = div_up(p->nx, kFaTileX), tiles_y = div_up(p->ny, ty);
         const size_t ntiles = static_cast<size_t>(tiles_x) * tiles_y;
-        // View segments per tile: enough CTAs for one image to fill the GPU
-        // (3 per SM).  A function of the geometry and device only, so an image's
-        // sums are the same in any batch.
+        // View segments per tile, summed in order.  A function of the geometry and
+        // device only, so an image's sums are the same in any batch.  More CTAs even
+        // out the last of them: with one launch of 3 segments 512^2 left three CTAs
+        // on some SMs and two on others (gather 175 -> 142 us in 8), 1024^2 three and
+        // four (call 1257 -> 990 us in 4).  Fewer where a segment's CTAs are many:
+        // 768^2 x 900 views 557 us in 6 and 570 in 8, 4 images of 2048^2 x 360 views
+        // 2583 in 2 and 2674 in 6.
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        int segs = static_cast<int>(std::max<size_t>(1, std::min<size_t>(8, 3ull * sms / ntiles)));
+        const size_t per_sm = ntiles / sms;
+        int segs = per_sm < 1 ? 8 : (per_sm < 3 ? 6 : (per_sm < 10 ? 4 : 2));
         const int seg_len = div_up(div_up(static_cast<int>(p->na), segs), kFaViews) * kFaViews;
         segs = div_up(static_cast<int>(p->na), seg_len);
         // tables of the call: fixed-point begin per (view, line), AdjView per
@@ -1844,21 +1876,30 @@ int fp_adjoint(const ctr_par_param* p, const T* proj, T* img, const double* w,
         const size_t nv = sizeof(AdjView) * p->na;
         const size_t nw = sizeof(AdjWin) * p->na * ntiles;
         const size_t part_at = (nb + nv + nw + 255) / 256 * 256;
-        const size_t npart = segs > 1 ? sizeof(float) * segs * batch * c.img_stride : 0;
+        // All segments at once, with partial images, while a segment's CTAs leave
+        // SMs idle (64^2 x 96 views: 135 against 153 us); else a launch a segment,
+        // which starts while the one before it ends (16 images of 512^2: 1446
+        // against 1562 us, and no partial images).
+        const bool parts = segs > 1 && div_up(batch, kImg) * ntiles < static_cast<size_t>(sms);
+        const size_t npart = parts ? sizeof(float) * segs * batch * c.img_stride : 0;
         void* scratch = nullptr;
         cudaError_t e = cudaMallocAsync(&scratch, part_at + npart, stream);
         if (e != cudaSuccess) return fail(CTR_ERR_CUDA, "fp_par_2d_grad scratch: %s", cudaGetErrorString(e));
         long long* B = static_cast<long long*>(scratch);
         AdjView* V = reinterpret_cast<AdjView*>(static_cast<char*>(scratch) + nb);
         AdjWin* W = reinterpret_cast<AdjWin*>(static_cast<char*>(scratch) + nb + nv);
-        float* part = segs > 1 ? reinterpret_cast<float*>(static_cast<char*>(scratch) + part_at) : nullptr;
+        float* part = parts ? reinterpret_cast<float*>(static_cast<char*>(scratch) + part_at) : nullptr;
         fp_adj_prep<<<div_up(static_cast<unsigned long long>(p->na) * p->nx, 256), 256, 0, stream>>>(
             w, pos, usex, B, V, p->na, p->nx);
         fp_adj_windows<<<div_up(static_cast<unsigned long long>(p->na) * std::max(tiles_x, tiles_y) * 32, 256),
                          256, 0, stream>>>(B, V, W, p->na, p->nx, tiles_x, tiles_y, ty, win);
-        fp_adj_launch<kRows, kImg>(proj, img, B, V, W, pos, c, tiles_x, tiles_y, batch, segs, seg_len, part,
-                                   stream);
-        if (segs > 1) {
+        e = fp_adj_launch<kRows, kImg>(proj, img, B, V, W, pos, c, tiles_x, tiles_y, batch, segs, seg_len, part,
+                                       stream);
+        if (e != cudaSuccess) {
+            cudaFreeAsync(scratch, stream);
+            return fail(CTR_ERR_CUDA, "fp_par_2d_grad: %s", cudaGetErrorString(e));
+        }
+        if (parts) {
             const size_t count = static_cast<size_t>(batch) * c.img_stride;
             const bool vec = count % 4 == 0 && reinterpret_cast<uintptr_t>(img) % 16 == 0;
             const unsigned blocks = static_cast<unsigned>(
