@@ -887,7 +887,8 @@ __global__ void __launch_bounds__(32 * kH8Warps, 8)
                 for (int r = 0; r < NR; ++r)  // 0 past the window
                     c[r] = fmaf(w, ldg_above_n(p + r * ns, t.n, r), cf.v * ldg_above_n(q + r * ns, t.n, r));
             };
-            if (held_n >= t.n && held == t.at - view) {
+            // (a longer one only where the lane's rows are taken one by one)
+            if ((t.out ? held_n >= t.n : held_n == t.n) && held == t.at - view) {
 #pragma unroll
                 for (int r = 0; r < NR; ++r) leftv[r] = right[r];
             } else {

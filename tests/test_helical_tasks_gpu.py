@@ -18,10 +18,22 @@ pytestmark = pytest.mark.gpu
     (129, 12, 200, 5, 1.0, 0.0), (200, 64, 97, 20, 0.45, 1.25),
     (290, 16, 330, 20, 1.0, 1.0), (321, 20, 257, 23, 0.8, 2.5), (257, 16, 300, 24, 0.9, 0.0)])
 def test_helical_groups(port, method, ns, nt, vpr, nz, pitch, thickness):
+    _check(port, method, ns, nt, vpr, nz, pitch, thickness, 1.0)
+
+
+@pytest.mark.parametrize("method", ["360", "180"])
+@pytest.mark.parametrize("ns,nt,vpr,nz,pitch,thickness", [
+    (290, 16, 330, 20, 1.0, 1.0), (321, 20, 257, 23, 0.8, 2.5), (257, 16, 300, 24, 0.9, 0.0), (300, 24, 400, 24, 0.5, 1.4)])
+def test_helical_couch_backwards(port, method, ns, nt, vpr, nz, pitch, thickness):
+    """The slab's rows move the other way from view to view."""
+    _check(port, method, ns, nt, vpr, nz, pitch, thickness, -1.0)
+
+
+def _check(port, method, ns, nt, vpr, nz, pitch, thickness, sign):
     from oracle import Heli
     from ct_recon_extensions_gb300 import torch_ctrecon as tc
     dso, dsd = 595.0, 1085.6
-    cm = pitch * nt * dso / dsd / vpr
+    cm = sign * pitch * nt * dso / dsd / vpr
     na = 4 * vpr
     h = Heli.make(ns=ns, nt=nt, na=na, ds=900.0 / ns, dt=1.0, view_per_rot=vpr, couch_mov=cm, nz=nz,
                   dz=1.7 * vpr * cm / nz, z0=(vpr + 3.3) * cm, thickness=thickness, dso=dso, dsd=dsd, offset_s=0.375,
