@@ -734,10 +734,13 @@ __global__ void __launch_bounds__(32 * kH3Warps, 12)
 // the interpolated rows out.  Detector rows are decided as in helical_360_f32;
 // a lane's complementary edges also depend on its fraction of dif.  A view's
 // rows are kept as a window of NR registers a lane, of which it sums its own.
-// Issue bound: 128 slices x 1152 views x 736 channels 1815 -> 1221 us.  With each
+// 128 slices x 1152 views x 736 channels: 1815 -> 1167 us, issue at 70 % of the slots:
+// the complementary samples take 630 us of them, the measured ones 340 (two views
+// at a time; 410 one by one, 8 at a time spill: 1305 us in all).  With each
 // lane's sums formed from memory instead of a window 1523 us, a branch per row
-// count 1280 us, 64 views a warp 1660 us, 10 blocks an SM spilled.
-constexpr int kH8Views = 32, kH8Warps = 4;
+// count 1280 us, the next window's loads a step ahead 1294 us (spills), 64 views
+// a warp 1660 us, 10 blocks an SM spilled.
+constexpr int kH8Views = 32, kH8Warps = 4, kH8Group = 2;
 static_assert(kH8Views == 32, "a view a lane, a lane's views in a 32-bit mask");
 
 template <int NR>
@@ -801,40 +804,68 @@ __global__ void __launch_bounds__(32 * kH8Warps, 8)
         return fminf(fabsf(dt), fabsf(db)) < guard;
     };
 
-    // 1. the measured samples
+    // 1. the measured samples, G views at a time (a view alone waits for its loads)
     {
+        constexpr int G = kH8Group;
+        int kind = 0;  // 1 rows that every lane uses, 2 lanes differ at an edge, 3 left
         if (lane < nv) {
             const HeliRowF& r = rows[iv0 + lane];
             H3View t;
             decide(r.at, r.ab, g0, g1, 0.0f, r.cur, t);
+            kind = t.n == -2 ? 3 : t.n < 0 ? 0 : t.out ? 2 : t.n > 0 ? 1 : 0;
             t.w = t.n > 0 ? __fdividef(1.0f, static_cast<float>(t.n)) : 0.0f;
             s_task[lane] = t;
             s_zd[lane] = r.zd;
         }
+        unsigned m_rows = __ballot_sync(0xffffffffu, kind == 1), m_mixed = __ballot_sync(0xffffffffu, kind == 2);
+        left |= __ballot_sync(0xffffffffu, kind == 3);
+        has = m_rows;
         __syncwarp();
-        for (int v = 0; v < nv; ++v) {
-            const H3View t = s_task[v];
-            if (t.n == -2) {
-                left |= 1u << v;
-                continue;
+        // the next views of a class, the last one again where there are fewer
+        auto take = [](unsigned& m, int (&k)[G]) {
+#pragma unroll
+            for (int u = 0; u < G; ++u) {
+                k[u] = __ffs(m) - 1;
+                const unsigned rest = m & (m - 1);
+                if (u == G - 1 || rest) m = rest;
             }
-            if (t.n == -1) continue;
-            bool any = true;
-            const unsigned at = t.at + is;
-            float m = (ldg_above<0>(in + at, t.n) + ldg_above<1>(in + (at + ns), t.n)) +
-                      (ldg_above<2>(in + (at + 2 * ns), t.n) + ldg_above<3>(in + (at + 3 * ns), t.n));
-            for (int r = 4; r < t.n; ++r) m += __ldg(in + (at + r * ns));
-            if (t.out) {
+        };
+        auto sum = [&](unsigned at, int n) {
+            float m = (ldg_above<0>(in + at, n) + ldg_above<1>(in + (at + ns), n)) +
+                      (ldg_above<2>(in + (at + 2 * ns), n) + ldg_above<3>(in + (at + 3 * ns), n));
+            for (int r = 4; r < n; ++r) m += __ldg(in + (at + r * ns));
+            return m;
+        };
+        while (m_rows) {
+            int k[G];
+            float m[G];
+            take(m_rows, k);
+#pragma unroll
+            for (int u = 0; u < G; ++u) {
+                const H3View& t = s_task[k[u]];
+                m[u] = t.w * sum(t.at + is, t.n);
+            }
+#pragma unroll
+            for (int u = 0; u < G; ++u) s_val[k[u] * 32 + lane] = m[u];
+        }
+        while (m_mixed) {
+            int k[G];
+            float m[G];
+            take(m_mixed, k);
+#pragma unroll
+            for (int u = 0; u < G; ++u) {
+                const H3View t = s_task[k[u]];
+                const unsigned at = t.at + is;
                 bool above, below;
-                if (extra(t, cf.g, 0.0f, above, below)) left |= 1u << v;
-                m += ldg_above<0>(in + (at - ns), above) + ldg_above<0>(in + (at + t.n * ns), below);
-                any = t.n + above + below > 0;
-                m = __fdividef(m, static_cast<float>(t.n + above + below));
-            } else {
-                m *= t.w;
+                if (extra(t, cf.g, 0.0f, above, below)) left |= 1u << k[u];
+                const int n = t.n + above + below;
+                m[u] = sum(at, t.n) +
+                       (ldg_above<0>(in + (at - ns), above) + ldg_above<0>(in + (at + t.n * ns), below));
+                m[u] = __fdividef(m[u], static_cast<float>(n));
+                has |= n > 0 ? 1u << k[u] : 0u;
             }
-            has |= any ? 1u << v : 0u;
-            s_val[v * 32 + lane] = m;
+#pragma unroll
+            for (int u = 0; u < G; ++u) s_val[k[u] * 32 + lane] = m[u];
         }
         __syncwarp();
     }
