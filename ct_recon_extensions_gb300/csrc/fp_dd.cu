@@ -544,6 +544,33 @@ __global__ void __launch_bounds__(256)
                            static_cast<float>(l), 0.5f * static_cast<float>(weights[ia]), (usex[ia] ? kDgUx : 0) | (ok ? 0 : kDgBad)};
 }
 
+// A pixel-view by itself, for any view: whether it adds anything, its first
+// channel, their count and the footprint's ends relative to the first, from
+// integers (in FP64 within 2^-16 of the row's start, and for views not of
+// DdView's form).
+__device__ __forceinline__ bool dd_grad_one(const DdView& v, const double* __restrict__ pp, int ix, int iy, int n,
+                                            long long room, int& first, int& cnt, float& lr, float& rr)
+{
+    const bool ux = v.flags & kDgUx;
+    const int along = ux ? ix : iy, line = ux ? iy : ix;
+    const long long mid = v.b + along * v.o + line * v.l;
+    long long left = along == 0 ? mid : mid - v.o, right = along == n - 1 ? mid : mid + v.o;
+    if (left > right) {
+        const long long t = left;
+        left = right;
+        right = t;
+    }
+    const long long c = (left + kDdHalf) >> 32;  // the left end's cell
+    first = static_cast<int>(c);
+    cnt = static_cast<int>(((right + kDdHalf) >> 32) - c) + 1;
+    lr = static_cast<float>(left - (c << 32)) * 2.3283064365386963e-10f;
+    rr = static_cast<float>(right - (c << 32)) * 2.3283064365386963e-10f;
+    const long long past = left + kDdHalf;  // > 0: the view counts (tie: decided in FP64)
+    if ((v.flags & kDgBad) || (past > -(1ll << 16) && past < (1ll << 16)))
+        return dd_grad_decide64(pp, ux, ix, iy, n, n, room, first, cnt, lr, rr);
+    return past > 0;
+}
+
 // A view on a tile.
 enum DgMode { kDgSkip, kDgInside, kDgEdge, kDgSlow };
 struct DgRec {
@@ -573,7 +600,12 @@ __device__ __forceinline__ DgRec dg_record(const DdView& v, int tx0, int ty0, in
     const float e = fabsf(r.sx) * (kDgTileX / 2) + fabsf(r.sy) * (kDgTileY / 2) + 0.51f;
     const float start = -0.5f - fmaxf(fminf(static_cast<float>(kc), 1e6f), -1e6f);  // channel -1/2, from the centre
     r.limit = start + (2.0f * r.reach - 1.0f);
-    if ((v.flags & kDgBad) || !(e + r.reach < kDgHalf - 3) || kc <= -1000000 || kc >= 0x40000000)
+    // A view whose lines run across its channels (angles outside [0, 2 pi) are
+    // not folded) has footprints narrow beside the tile, and a weight to match:
+    // positions within the tile in FP32 would cost it digits (5e-5 of the peak
+    // against 3e-7).
+    const bool across = fabsf(v.lf) > 2.0f * r.reach;
+    if ((v.flags & kDgBad) || across || !(e + r.reach < kDgHalf - 3) || kc <= -1000000 || kc >= 0x40000000)
         r.mode = kDgSlow;
     else if (e < start - 0.01f)
         r.mode = kDgSkip;
@@ -666,22 +698,22 @@ __global__ void __launch_bounds__(kDgThreads, 3)
             if (r.mode == kDgSkip) continue;
             if (r.mode == kDgSlow) {
                 const long long row = static_cast<long long>(v0 + j) * ns;
-                const bool ux = r.flags & kDgUx;
+                const DdView v = views[v0 + j];
                 for (int k = 0; k < kDgRows; ++k) {
                     const int iy = iy0 + k;
                     int first, cnt;
                     float lr, rr, t = 0.0f;
                     if (ix < n && iy < n &&
-                        dd_grad_decide64(pos + static_cast<size_t>(v0 + j) * n * 2, ux, ix, iy, n, n, total - 1 - row,
-                                         first, cnt, lr, rr))
+                        dd_grad_one(v, pos + static_cast<size_t>(v0 + j) * n * 2, ix, iy, n, total - 1 - row, first, cnt,
+                                    lr, rr))
                         for (int c = 0; c < cnt; ++c) {
                             const float fc = static_cast<float>(c);
                             const float len = fminf(fc + 0.5f, rr) - fmaxf(fc - 0.5f, lr);
-                            t = fmaf(len, __ldg(P + row + first + c), t);
+                            if (first + c >= 0 && row + first + c < total) t = fmaf(len, __ldg(P + row + first + c), t);
                         }
 #pragma unroll
                     for (int q = 0; q < kDgRows; ++q)  // blk stays in registers
-                        if (q == k) blk[q] = fmaf(t, views[v0 + j].half_w, blk[q]);
+                        if (q == k) blk[q] = fmaf(t, v.half_w, blk[q]);
                 }
                 continue;
             }
@@ -753,26 +785,10 @@ __global__ void __launch_bounds__(kDbThreads)
     float sum = 0.0f;
     for (int ia = warp; ia < na; ia += kDbThreads / 32) {
         const DdView v = views[ia];
-        const bool ux = v.flags & kDgUx;
-        const int along = ux ? ix : iy, line = ux ? iy : ix;
         const long long row = static_cast<long long>(ia) * ns;
-        const long long mid = v.b + along * v.o + line * v.l;
-        long long left = along == 0 ? mid : mid - v.o, right = along == n - 1 ? mid : mid + v.o;
-        if (left > right) {
-            const long long t = left;
-            left = right;
-            right = t;
-        }
-        const long long c = (left + kDdHalf) >> 32;  // the left end's cell
-        int first = static_cast<int>(c), cnt = static_cast<int>(((right + kDdHalf) >> 32) - c) + 1;
-        float lr = static_cast<float>(left - (c << 32)) * 2.3283064365386963e-10f;
-        float rr = static_cast<float>(right - (c << 32)) * 2.3283064365386963e-10f;
-        const long long past = left + kDdHalf;  // > 0: the view counts (tie: decided in FP64)
-        bool on = past > 0;
-        if ((v.flags & kDgBad) || (past > -(1ll << 16) && past < (1ll << 16)))
-            on = dd_grad_decide64(pos + static_cast<size_t>(ia) * n * 2, ux, ix, iy, n, n, total - 1 - row, first, cnt,
-                                  lr, rr);
-        if (!on) continue;
+        int first, cnt;
+        float lr, rr;
+        if (!dd_grad_one(v, pos + static_cast<size_t>(ia) * n * 2, ix, iy, n, total - 1 - row, first, cnt, lr, rr)) continue;
         float t = 0.0f;
         for (int k = 0; k < cnt; ++k) {
             const long long at = row + first + k;
