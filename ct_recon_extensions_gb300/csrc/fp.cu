@@ -1192,7 +1192,7 @@ __device__ __forceinline__ void adj_tap_staged(float (&blk)[IMG][ROWS], int r, l
 // the windows' pairs (all loads in flight), one barrier, compute, one barrier;
 // the next block's view constants and windows are copied (cp.async) during
 // the compute into the other half of s_v / s_w.
-template <int ROWS, int IMG>
+template <int ROWS, int IMG, bool ADD>
 __global__ void __launch_bounds__(256, ROWS * IMG >= 32 ? 2 : 3)
     fp_adj_f32(const float* __restrict__ proj, float* __restrict__ img, const long long* __restrict__ B,
                const AdjView* __restrict__ V, const AdjWin* __restrict__ W, const double* __restrict__ pos,
@@ -1332,8 +1332,7 @@ __global__ void __launch_bounds__(256, ROWS * IMG >= 32 ? 2 : 3)
         cp_async_wait_all();
         __syncthreads();
     }
-    const bool add = split == 1 && seg0 > 0;
-    if (add) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if constexpr (ADD) asm volatile("griddepcontrol.wait;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < IMG; ++i) {
         float* O = split == 1 ? img + static_cast<size_t>(im + i) * c.img_stride
@@ -1343,7 +1342,7 @@ __global__ void __launch_bounds__(256, ROWS * IMG >= 32 ? 2 : 3)
             const int iy = ty0 + warp * ROWS + r;
             if (ix < c.nx && iy < c.ny) {
                 float* o = O + static_cast<size_t>(iy) * c.nx + ix;
-                *o = add ? *o + acc[i][r] : acc[i][r];
+                *o = ADD ? *o + acc[i][r] : acc[i][r];
             }
         }
     }
@@ -1689,9 +1688,10 @@ int launch_fpx_proj(const FpxConst& c, size_t smem, const FpxRays& r, const floa
     if (e != cudaSuccess) return fail(CTR_ERR_CUDA, "fp smem: %s", cudaGetErrorString(e));
     // Pairs of images (1165 against 1680 us for 16 of 512^2), where both bands of
     // 16 rows fit a stage (n <= 512) and their rows start alike in 16 bytes (even
-    // n); the last one of an odd batch by itself.
+    // n); the last one of an odd batch by itself.  Below 64^2 a call is its
+    // launches: 5 images of 32^2 19 us in one, 23 in two.
     int done = 0;
-    if (batch > 1 && c.n <= 512 && c.n % 2 == 0) {
+    if (batch > 1 && c.n >= 64 && c.n <= 512 && c.n % 2 == 0) {
         const FpxKernel pair = fp_proj_f32<16, 2>;
         constexpr size_t smem2 = 128 + sizeof(float) * kFpxStages * 2 * kFpxSecond;
         FpxConst c2 = c;
@@ -1810,9 +1810,7 @@ cudaError_t fp_adj_launch(const float* proj, float* img, const long long* B, con
 {
     constexpr size_t smem = sizeof(float) * kFaViews * FaShape<ROWS>::WIN * 2 * IMG;
     constexpr size_t smem1 = sizeof(float) * kFaViews * FaShape<ROWS>::WIN * 2;
-    if (smem > 48 * 1024)  // above the default limit (set per call: the current device's)
-        cudaFuncSetAttribute(fp_adj_f32<ROWS, IMG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem));
+    static_assert(smem <= 48 * 1024, "within the default limit");
     cudaLaunchAttribute early{};
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     early.val.programmaticStreamSerializationAllowed = 1;
@@ -1823,21 +1821,22 @@ cudaError_t fp_adj_launch(const float* proj, float* img, const long long* B, con
     cudaError_t e = cudaSuccess;
     // `count` CTAs' images from img0 on: every segment in one launch (part), or a
     // launch a segment, each but the first adding to the one before it
-    auto launch = [&](auto kern, size_t bytes, int img0, int count) {
+    auto launch = [&](auto first, auto add, size_t bytes, int img0, int count) {
         const int split = part ? segs : 1;
         cfg.dynamicSmemBytes = bytes;
         cfg.gridDim = dim3(tiles_x, tiles_y, count * split);
         for (int seg = 0; seg < segs && e == cudaSuccess; seg += split) {
             cfg.numAttrs = seg > 0 ? 1 : 0;
-            e = cudaLaunchKernelEx(&cfg, kern, proj, img, B, V, W, pos, c, img0, split, seg, seg_len, part, batch);
+            e = cudaLaunchKernelEx(&cfg, seg > 0 ? add : first, proj, img, B, V, W, pos, c, img0, split, seg, seg_len,
+                                   part, batch);
         }
     };
     const int groups = batch / IMG, zmax = 65535 / segs;
     for (int g0 = 0; g0 < groups; g0 += zmax)
-        launch(fp_adj_f32<ROWS, IMG>, smem, g0 * IMG, std::min(zmax, groups - g0));
+        launch(fp_adj_f32<ROWS, IMG, false>, fp_adj_f32<ROWS, IMG, true>, smem, g0 * IMG, std::min(zmax, groups - g0));
     if constexpr (IMG > 1) {
         const int rest = batch - groups * IMG;
-        if (rest > 0) launch(fp_adj_f32<ROWS, 1>, smem1, groups * IMG, rest);
+        if (rest > 0) launch(fp_adj_f32<ROWS, 1, false>, fp_adj_f32<ROWS, 1, true>, smem1, groups * IMG, rest);
     }
     return e;
 }
@@ -1868,6 +1867,8 @@ int fp_adjoint(const ctr_par_param* p, const T* proj, T* img, const double* w,
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const size_t per_sm = ntiles / sms;
         int segs = per_sm < 1 ? 8 : (per_sm < 3 ? 6 : (per_sm < 10 ? 4 : 2));
+        // (at least 32 views each where the tiles alone give half of the SMs a CTA)
+        if (2 * ntiles >= static_cast<size_t>(sms)) segs = std::min(segs, std::max(1, static_cast<int>(p->na) / 32));
         const int seg_len = div_up(div_up(static_cast<int>(p->na), segs), kFaViews) * kFaViews;
         segs = div_up(static_cast<int>(p->na), seg_len);
         // tables of the call: fixed-point begin per (view, line), AdjView per
@@ -1877,13 +1878,19 @@ int fp_adjoint(const ctr_par_param* p, const T* proj, T* img, const double* w,
         const size_t nw = sizeof(AdjWin) * p->na * ntiles;
         const size_t part_at = (nb + nv + nw + 255) / 256 * 256;
         // All segments at once, with partial images, while a segment's CTAs leave
-        // SMs idle (64^2 x 96 views: 135 against 153 us); else a launch a segment,
-        // which starts while the one before it ends (16 images of 512^2: 1446
-        // against 1562 us, and no partial images).
-        const bool parts = segs > 1 && div_up(batch, kImg) * ntiles < static_cast<size_t>(sms);
-        const size_t npart = parts ? sizeof(float) * segs * batch * c.img_stride : 0;
+        // SMs idle (64^2 x 96 views: 135 against 153 us) or are short (5 images of
+        // 512^2 x 90 views: 106 against 123 us); else, and where there is no room for
+        // the partial images, a launch a segment, which starts while the one before
+        // it ends (16 images of 512^2: 1446 against 1562 us).
+        bool parts = segs > 1 && (div_up(batch, kImg) * ntiles < static_cast<size_t>(sms) || seg_len <= 48);
+        const size_t npart = sizeof(float) * segs * batch * c.img_stride;
         void* scratch = nullptr;
-        cudaError_t e = cudaMallocAsync(&scratch, part_at + npart, stream);
+        cudaError_t e = cudaMallocAsync(&scratch, part_at + (parts ? npart : 0), stream);
+        if (e == cudaErrorMemoryAllocation && parts) {
+            cudaGetLastError();
+            parts = false;
+            e = cudaMallocAsync(&scratch, part_at, stream);
+        }
         if (e != cudaSuccess) return fail(CTR_ERR_CUDA, "fp_par_2d_grad scratch: %s", cudaGetErrorString(e));
         long long* B = static_cast<long long*>(scratch);
         AdjView* V = reinterpret_cast<AdjView*>(static_cast<char*>(scratch) + nb);
