@@ -851,13 +851,22 @@ int dd_forward(const ctr_par_param* p, const T* img, T* proj, const double* sc, 
         if (batch > 65535) return fail(CTR_ERR_UNSUPPORTED, "batch > 65535");
         float* rows = nullptr;
         const size_t copy = static_cast<size_t>(n) * (n + kDdPad);
-        cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&rows), 2 * sizeof(float) * copy * batch, stream);
+        int most = batch;  // images at a time: fewer where there is no room for every one's copies
+        cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&rows), 2 * sizeof(float) * copy * most, stream);
+        while (e == cudaErrorMemoryAllocation && most > 1) {
+            cudaGetLastError();
+            most = (most + 1) / 2;
+            e = cudaMallocAsync(reinterpret_cast<void**>(&rows), 2 * sizeof(float) * copy * most, stream);
+        }
         if (e != cudaSuccess) return fail(CTR_ERR_CUDA, "distance-driven scratch: %s", cudaGetErrorString(e));
-        float* cols = rows + copy * batch;
         const unsigned tiles = div_up(n + kDdPad, 32), chunks = div_up(p->ns, kDdRayThreads);
-        dd_copies<<<dim3(tiles, tiles, batch), 256, 0, stream>>>(img, rows, cols, n);
-        fp_dd_f32<<<dim3(chunks * p->na, batch), kDdRayThreads, 0, stream>>>(
-            img, rows, cols, proj, sc, bo, usex, p->ns, chunks, n, p->dx, p->dy, is, ps);
+        for (int i = 0; i < batch; i += most) {
+            const int count = std::min(most, batch - i);
+            float* cols = rows + copy * count;
+            dd_copies<<<dim3(tiles, tiles, count), 256, 0, stream>>>(img + i * is, rows, cols, n);
+            fp_dd_f32<<<dim3(chunks * p->na, count), kDdRayThreads, 0, stream>>>(
+                img + i * is, rows, cols, proj + i * ps, sc, bo, usex, p->ns, chunks, n, p->dx, p->dy, is, ps);
+        }
         st = check_launch("fp_par_2d distance driven");
         cudaFreeAsync(rows, stream);  // after the kernel that reads it
         return st;
