@@ -976,6 +976,7 @@ struct FaShape {
     static constexpr int TY = 8 * ROWS;
     static constexpr int LINES = TY > kFaTileX ? TY : kFaTileX;  // rows or columns of a tile
     static constexpr int WIN = 2 * LINES;                        // staged channel pairs per view
+    static constexpr int RAW = WIN + 4;                          // channels copied per view (WIN + 1)
 };
 // Units of 2^-32 channel within which a border pixel's position counts as on a
 // channel: the fixed-point position is within 0.5 + 0.5*along units of the
@@ -1182,16 +1183,25 @@ __device__ __forceinline__ void adj_tap_staged(float (&blk)[IMG][ROWS], int r, l
     }
 }
 
+// The float at src, or 0 (src is not read).
+__device__ __forceinline__ void cp_async4_or_zero(unsigned dst, const float* src, bool read)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(read ? 4 : 0) : "memory");
+}
+
 // The gather: CTA = one 32 x 8*ROWS tile of IMG images and one segment of
 // seg_len views: blockIdx.z = group * split + k for segment seg0 + k, images img0 +
 // group*IMG ...  With split == 1 it writes the images (seg0 == 0) or adds to them
 // what the launches of the segments before it have written; with several, segment
 // s writes its partial sums to part[s][image] for fp_adj_reduce.  A launch that
 // adds may start while the one before it ends (its CTAs fill the SMs that run
-// dry); it waits for that one where it first reads the images.  Per block of kFaViews views: one phase loads the tile's line positions and
-// the windows' pairs (all loads in flight), one barrier, compute, one barrier;
-// the next block's view constants and windows are copied (cp.async) during
-// the compute into the other half of s_v / s_w.
+// dry); it waits for that one where it first reads the images.  Per block
+// of kFaViews views: its line positions and its windows' channels arrive (cp.async,
+// issued during the block before it, with the view constants and windows of the
+// block after it), a barrier, the channels become pairs, a warp a view, a barrier,
+// compute.  The copies loaded through registers at the block's start cost their
+// latency: 141 -> 133 us for one 512^2 image of 720 views, 16 images 1435 -> 1398
+// (call); two views a warp's pass over the whole window's length 138.
 template <int ROWS, int IMG, bool ADD>
 __global__ void __launch_bounds__(256, ROWS * IMG >= 32 ? 2 : 3)
     fp_adj_f32(const float* __restrict__ proj, float* __restrict__ img, const long long* __restrict__ B,
@@ -1199,13 +1209,14 @@ __global__ void __launch_bounds__(256, ROWS * IMG >= 32 ? 2 : 3)
                const FpConst c, int img0, int split, int seg0, int seg_len, float* __restrict__ part, int batch)
 {
     using S = FaShape<ROWS>;
-    constexpr int TY = S::TY, LINES = S::LINES, WIN = S::WIN;
+    constexpr int TY = S::TY, LINES = S::LINES, WIN = S::WIN, RAW = S::RAW;
     static_assert(IMG == 1 || IMG == 2 || IMG == 4, "images per CTA");
-    __shared__ long long s_base[kFaViews][LINES];
-    __shared__ AdjView s_v[2][kFaViews];
-    __shared__ AdjWin s_w[2][kFaViews];
-    extern __shared__ __align__(16) float s_pair_dyn[];  // [kFaViews][WIN][2 * IMG]
+    __shared__ long long s_base[2][kFaViews][LINES];
+    __shared__ AdjView s_v[3][kFaViews];
+    __shared__ AdjWin s_w[3][kFaViews];
+    extern __shared__ __align__(16) float s_pair_dyn[];  // [kFaViews][WIN][2 * IMG], then [kFaViews][IMG][RAW]
     float(*s_pair)[WIN][2 * IMG] = reinterpret_cast<float(*)[WIN][2 * IMG]>(s_pair_dyn);
+    float(*s_raw)[IMG][RAW] = reinterpret_cast<float(*)[IMG][RAW]>(s_pair_dyn + kFaViews * WIN * 2 * IMG);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1223,74 +1234,97 @@ __global__ void __launch_bounds__(256, ROWS * IMG >= 32 ? 2 : 3)
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) acc[i][r] = 0.0f;
 
-    if (tid < min(kFaViews, ve - vb)) {
-        s_v[0][tid] = V[vb + tid];
-        s_w[0][tid] = W[static_cast<size_t>(vb + tid) * ntiles + tile];
+    if (tid < min(2 * kFaViews, ve - vb)) {
+        s_v[tid / kFaViews][tid % kFaViews] = V[vb + tid];
+        s_w[tid / kFaViews][tid % kFaViews] = W[static_cast<size_t>(vb + tid) * ntiles + tile];
     }
     __syncthreads();
-    int buf = 0;
-    for (int v0 = vb; v0 < ve; v0 += kFaViews, buf ^= 1) {
+    // Copies of the block of views from v0 on (cp.async): the tile's line positions
+    // (rows for row-marching views, else columns) and the windows' channels, zero
+    // off the detector
+    auto fetch = [&](int v0, int v3, int base) {
         const int nv = min(kFaViews, ve - v0);
-        // the next block's view constants and windows, copied during this
-        // block into the other half of s_v / s_w (last read before this
-        // block's first barrier)
-        const int vn = v0 + kFaViews + tid;
-        if (tid < kFaViews && vn < ve) {
-            static_assert(sizeof(AdjView) == 24 && sizeof(AdjWin) == 8, "8-byte copies");
-            const unsigned dv = smem_u32(&s_v[buf ^ 1][tid]);
-            const char* sv = reinterpret_cast<const char*>(V + vn);
-            cp_async8(dv, sv);
-            cp_async8(dv + 8, sv + 8);
-            cp_async8(dv + 16, sv + 16);
-            cp_async8(smem_u32(&s_w[buf ^ 1][tid]), W + static_cast<size_t>(vn) * ntiles + tile);
-        }
-        // line positions of the tile: rows for row-marching views, else columns
 #pragma unroll
         for (int it = 0; it < kFaViews * LINES / 256; ++it) {
             const int idx = it * 256 + tid;
             const int j = idx / LINES, l = idx - j * LINES;
             if (j < nv) {
-                const int ux = s_v[buf][j].ux;
+                const int ux = s_v[v3][j].ux;
                 if (l < (ux ? TY : kFaTileX))
-                    s_base[j][l] = __ldg(B + static_cast<size_t>(v0 + j) * n + min((ux ? ty0 : tx0) + l, n - 1));
+                    cp_async8(smem_u32(&s_base[base][j][l]),
+                              B + static_cast<size_t>(v0 + j) * n + min((ux ? ty0 : tx0) + l, n - 1));
             }
         }
-        // staged windows: (w p[lo+k], w p[lo+k+1]) per image, zero off the detector
 #pragma unroll
-        for (int it = 0; it < kFaViews * WIN / 256; ++it) {
-            const int idx = it * 256 + tid;
-            const int j = idx / WIN, k = idx - j * WIN;
-            if (j < nv && k < s_w[buf][j].width) {
-                const float w = s_v[buf][j].w;
-                const int g = s_w[buf][j].lo + k;
-                const bool in0 = static_cast<unsigned>(g) < static_cast<unsigned>(ns);
-                const bool in1 = static_cast<unsigned>(g + 1) < static_cast<unsigned>(ns);
-                const float* row = P + static_cast<size_t>(v0 + j) * ns;
+        for (int h = 0; h < kFaViews / 8; ++h) {  // a warp a view
+            const int j = warp + 8 * h;
+            if (j >= nv || s_w[v3][j].width == 0) continue;
+            const int lo = s_w[v3][j].lo, width = s_w[v3][j].width;
+            const float* row = P + static_cast<size_t>(v0 + j) * ns;
+            for (int k = lane; k <= width; k += 32) {
+                const int g = lo + k;
+                const bool in = static_cast<unsigned>(g) < static_cast<unsigned>(ns);
+                const float* src = row + (in ? g : 0);
+#pragma unroll
+                for (int i = 0; i < IMG; ++i)
+                    cp_async4_or_zero(smem_u32(&s_raw[j][i][k]), src + i * c.proj_stride, in);
+            }
+        }
+    };
+    fetch(vb, 0, 0);
+    int v3 = 0, base = 0;  // buffers of this block
+    for (int v0 = vb; v0 < ve; v0 += kFaViews) {
+        const int nv = min(kFaViews, ve - v0);
+        cp_async_wait_all();
+        __syncthreads();  // this block's copies are there; every warp is done with the last block's pairs
+        // staged windows: (w p[lo+k], w p[lo+k+1]) per image
+#pragma unroll
+        for (int h = 0; h < kFaViews / 8; ++h) {
+            const int j = warp + 8 * h;
+            if (j >= nv) continue;
+            const int width = s_w[v3][j].width;
+            const float w = s_v[v3][j].w;
+            for (int k = lane; k < width; k += 32) {
                 float e[2 * IMG];
 #pragma unroll
                 for (int i = 0; i < IMG; ++i) {
-                    e[2 * i] = in0 ? __ldg(row + i * c.proj_stride + g) * w : 0.0f;
-                    e[2 * i + 1] = in1 ? __ldg(row + i * c.proj_stride + g + 1) * w : 0.0f;
+                    e[2 * i] = s_raw[j][i][k] * w;
+                    e[2 * i + 1] = s_raw[j][i][k + 1] * w;
                 }
                 if constexpr (IMG == 1) {
                     *reinterpret_cast<float2*>(&s_pair[j][k][0]) = make_float2(e[0], e[1]);
                 } else {
 #pragma unroll
-                    for (int h = 0; h < IMG / 2; ++h)
-                        *reinterpret_cast<float4*>(&s_pair[j][k][4 * h]) =
-                            make_float4(e[4 * h], e[4 * h + 1], e[4 * h + 2], e[4 * h + 3]);
+                    for (int q = 0; q < IMG / 2; ++q)
+                        *reinterpret_cast<float4*>(&s_pair[j][k][4 * q]) =
+                            make_float4(e[4 * q], e[4 * q + 1], e[4 * q + 2], e[4 * q + 3]);
                 }
             }
         }
         __syncthreads();
+        // the next block's copies during this block's sums, and the view constants
+        // and windows of the one after it
+        const int w3 = v3 == 2 ? 0 : v3 + 1;
+        if (v0 + kFaViews < ve) fetch(v0 + kFaViews, w3, base ^ 1);
+        const int vn = v0 + 2 * kFaViews + tid;
+        if (tid < kFaViews && vn < ve) {
+            static_assert(sizeof(AdjView) == 24 && sizeof(AdjWin) == 8, "8-byte copies");
+            const int x3 = w3 == 2 ? 0 : w3 + 1;
+            const unsigned dv = smem_u32(&s_v[x3][tid]);
+            const char* sv = reinterpret_cast<const char*>(V + vn);
+            cp_async8(dv, sv);
+            cp_async8(dv + 8, sv + 8);
+            cp_async8(dv + 16, sv + 16);
+            cp_async8(smem_u32(&s_w[x3][tid]), W + static_cast<size_t>(vn) * ntiles + tile);
+        }
         float blk[IMG][ROWS];  // this view block's partial sums (blocked summation)
 #pragma unroll
         for (int i = 0; i < IMG; ++i)
 #pragma unroll
             for (int r = 0; r < ROWS; ++r) blk[i][r] = 0.0f;
         for (int j = 0; j < nv; ++j) {
-            const AdjView v = s_v[buf][j];
-            const AdjWin wn = s_w[buf][j];
+            const AdjView v = s_v[v3][j];
+            const AdjWin wn = s_w[v3][j];
             if (wn.width > 0) {
                 const float inv1 = 1.0f - v.inv;
                 const unsigned pb = smem_u32(&s_pair[j][0][0]) - 8u * IMG * static_cast<unsigned>(wn.lo);
@@ -1298,9 +1332,9 @@ __global__ void __launch_bounds__(256, ROWS * IMG >= 32 ? 2 : 3)
                     const long long A = static_cast<long long>(ix) * v.O1;
 #pragma unroll
                     for (int r = 0; r < ROWS; ++r)
-                        adj_tap_staged<IMG, ROWS>(blk, r, s_base[j][warp * ROWS + r] + A, pb, v.inv, inv1);
+                        adj_tap_staged<IMG, ROWS>(blk, r, s_base[base][j][warp * ROWS + r] + A, pb, v.inv, inv1);
                 } else {     // along = row, line = ix
-                    long long MID = s_base[j][lane] + static_cast<long long>(ty0 + warp * ROWS) * v.O1;
+                    long long MID = s_base[base][j][lane] + static_cast<long long>(ty0 + warp * ROWS) * v.O1;
 #pragma unroll
                     for (int r = 0; r < ROWS; ++r) {
                         adj_tap_staged<IMG, ROWS>(blk, r, MID, pb, v.inv, inv1);
@@ -1313,7 +1347,7 @@ __global__ void __launch_bounds__(256, ROWS * IMG >= 32 ? 2 : 3)
                     const int iy = ty0 + warp * ROWS + r;
                     const int along = v.ux ? ix : iy;
                     const int lin = v.ux ? iy : ix;
-                    const long long MID = s_base[j][v.ux ? warp * ROWS + r : lane] +
+                    const long long MID = s_base[base][j][v.ux ? warp * ROWS + r : lane] +
                                           static_cast<long long>(along) * v.O1;
                     const double* pp = pos + (static_cast<size_t>(v0 + j) * n + min(lin, n - 1)) * 2;
                     const AdjTap t = adj_tap_plan(MID, v.O1, v.inv, v.two != 0, along, n, ns, pp);
@@ -1329,8 +1363,8 @@ __global__ void __launch_bounds__(256, ROWS * IMG >= 32 ? 2 : 3)
         for (int i = 0; i < IMG; ++i)
 #pragma unroll
             for (int r = 0; r < ROWS; ++r) acc[i][r] += blk[i][r];
-        cp_async_wait_all();
-        __syncthreads();
+        v3 = w3;
+        base ^= 1;
     }
     if constexpr (ADD) asm volatile("griddepcontrol.wait;" ::: "memory");
 #pragma unroll
@@ -1808,9 +1842,9 @@ cudaError_t fp_adj_launch(const float* proj, float* img, const long long* B, con
                           const double* pos, const FpConst& c, int tiles_x, int tiles_y, int batch, int segs,
                           int seg_len, float* part, cudaStream_t stream)
 {
-    constexpr size_t smem = sizeof(float) * kFaViews * FaShape<ROWS>::WIN * 2 * IMG;
-    constexpr size_t smem1 = sizeof(float) * kFaViews * FaShape<ROWS>::WIN * 2;
-    static_assert(smem <= 48 * 1024, "within the default limit");
+    constexpr size_t smem1 = sizeof(float) * kFaViews * (FaShape<ROWS>::WIN * 2 + FaShape<ROWS>::RAW), smem = smem1 * IMG;
+    cudaFuncSetAttribute(fp_adj_f32<ROWS, IMG, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaFuncSetAttribute(fp_adj_f32<ROWS, IMG, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     cudaLaunchAttribute early{};
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     early.val.programmaticStreamSerializationAllowed = 1;
