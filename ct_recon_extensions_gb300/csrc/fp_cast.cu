@@ -117,13 +117,13 @@ __global__ void __launch_bounds__(kCastThreads)
 // copy.  Both copies have a border of kCastPad zeros around the image (the
 // fixed-point positions may sit a hair outside it, where the weight is ~0), so
 // the loop has no clamps.  Issue bound: ~75 instructions per ray and row, 67 %
-// of the issue slots (512^2 x 720 x 729 at a step of 0.125: 2450 -> 411 us).
+// of the issue slots (512^2 x 720 x 729 at a step of 0.125: 2450 -> 388 us).
 // Blocks start with the long rays of every view, near the detector's middle, and
 // end with short ones: view by view the SMs ran dry one by one (467 us).
-// Blocks of 64 rays: 128 took as long, 32 were 2 % slower; fewer registers for
-// more warps spilled (20 blocks of 64 a SM: 526 us).
+// Blocks of 64 rays took 411 us, of 128 422; fewer registers for more warps
+// spilled (20 blocks of 64 a SM, view by view: 526 us).
 constexpr int kCastPad = 2;
-constexpr int kRowThreads = 64, kRowBlocks = 16;  // rays a block, blocks an SM
+constexpr int kRowThreads = 32, kRowBlocks = 32;  // rays a block, blocks an SM
 
 // The padded image and its padded transpose, 32 x 32 tiles of padded pixels.
 __global__ void __launch_bounds__(256)
@@ -309,7 +309,7 @@ int check_cast(const ctr_par_param* p, double step_size, const void* a, const vo
 // Steps up to this many pixels go row by row (fp_cast_rows_f32): the time does
 // not depend on the step there, that of the sample-by-sample kernel does.  Per
 // call (copies included), row by row against sample by sample:
-//   512^2 x 720 x 729   step 0.125: 411 / 2450 us, 0.5: 411 / 1176, 0.75: 411 / 1040
+//   512^2 x 720 x 729   step 0.125: 393 / 2450 us, 0.5: 393 / 1176, 0.75: 393 / 1040
 //   128^2 x 180 x 190   step 0.125: 51 / 135 us,   0.5: 41 / 57,    0.75: 40 / 45
 //   64^2 x 90 x 96      step 0.125: 34 / 70 us,    0.5: 30 / 33,    0.75: 31 / 28
 constexpr double kCastRowStep = 0.5;
