@@ -312,7 +312,11 @@ int check_cast(const ctr_par_param* p, double step_size, const void* a, const vo
 //   512^2 x 720 x 729   step 0.125: 393 / 2450 us, 0.5: 393 / 1176, 0.75: 393 / 1040
 //   128^2 x 180 x 190   step 0.125: 51 / 135 us,   0.5: 41 / 57,    0.75: 40 / 45
 //   64^2 x 90 x 96      step 0.125: 34 / 70 us,    0.5: 30 / 33,    0.75: 31 / 28
-constexpr double kCastRowStep = 0.5;
+// Geometries of fewer samples than kCastRowSamples (rays times the image's shorter
+// side in steps; an item's path is the same in any batch) are launches, of which the
+// copies are one more: 32^2 x 30 x 45 at a step of 0.25 23 / 19 us, 16^2 x 12 x 21
+// 21 / 15.
+constexpr double kCastRowStep = 0.5, kCastRowSamples = 5e5;
 constexpr int kCastNotRows = -1;
 
 // The row-by-row path of an FP32 call, kCastNotRows where it does not take it.
@@ -324,6 +328,7 @@ int cast_rows(const ctr_par_param* p, double step_size, const float* img, float*
     const size_t blocks = static_cast<size_t>(chunks) * p->na;
     // the march indexes a copy with 32-bit integers
     if (step_size > kCastRowStep || wx * wy > 0x7fffffffu || blocks > 0x7fffffffu) return kCastNotRows;
+    if (static_cast<double>(p->na) * p->ns * std::min(p->nx, p->ny) < kCastRowSamples * step_size) return kCastNotRows;
     float* rows = nullptr;
     const size_t item = wx * wy;
     if (cudaMallocAsync(reinterpret_cast<void**>(&rows), 2 * sizeof(float) * item * batch, stream) != cudaSuccess) {

@@ -17,7 +17,10 @@ pytestmark = pytest.mark.gpu
     (1, 1, 5, 4, 0.5, 0.1), (28, 28, 127, 8, 0.125, 0.0), (29, 60, 128, 9, 0.25, math.pi / 4),
     (61, 28, 129, 12, 0.01, 0.3), (33, 92, 257, 16, 0.5, 0.0), (92, 33, 50, 16, 0.51, 0.0),
     (64, 64, 65, 10, 0.37, 0.7), (31, 31, 64, 7, 1.0, 0.0),
-    (40, 40, 64, 7, 3.0, 0.2)])
+    (40, 40, 64, 7, 3.0, 0.2),
+    # enough samples for the rows
+    (1, 1, 31, 1700, 0.1, 0.1), (28, 28, 127, 20, 0.125, 0.0), (29, 60, 128, 36, 0.25, math.pi / 4),
+    (33, 92, 257, 32, 0.5, 0.0), (92, 33, 50, 160, 0.5, 0.0), (64, 64, 65, 48, 0.37, 0.7), (30, 30, 33, 130, 0.25, 0.2)])
 def test_cast_rows(port, nx, ny, ns, na, step, start):
     from oracle import Geom
     from ct_recon_extensions_gb300 import torch_ctrecon as tc
