@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "ctr_common.cuh"
+#include "dd_window.h"
 #include "fp_setup.cuh"
 
 namespace ctr {
@@ -520,7 +521,6 @@ __global__ void __launch_bounds__(kDdThreads)
 // kernels).  A running integral over the window, looked up at both ends, took
 // as long and lost the digits of small channels beside a large one.
 constexpr int kDgTileX = 32, kDgTileY = 64, kDgRows = 8, kDgViews = 16, kDgThreads = 256;
-constexpr int kDgHalf = 64;  // channels staged on either side of the window's centre
 constexpr float kDgMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer in the low bits
 
 // A view's positions: channel of pixel (along, line) = b + along * o + line * l.
@@ -612,14 +612,14 @@ __device__ __forceinline__ DgRec dg_record(const DdView& v, int tx0, int ty0, in
     // positions within the tile in FP32 would cost it digits (5e-5 of the peak
     // against 3e-7).
     const bool across = fabsf(v.lf) > 2.0f * r.reach;
-    if ((v.flags & kDgBad) || across || !(e + r.reach < kDgHalf - 3) || kc <= -1000000 || kc >= 0x40000000)
+    if ((v.flags & kDgBad) || across || !dg_fits(e, r.reach) || kc <= -1000000 || kc >= 0x40000000)
         r.mode = kDgSlow;
     else if (e < start - 0.01f)
         r.mode = kDgSkip;
     else
         r.mode = -e - r.reach > start + 0.01f ? kDgInside : kDgEdge;
     *centre = static_cast<int>(kc);
-    *need = r.mode == kDgInside || r.mode == kDgEdge ? static_cast<int>(e + r.reach) + 2 : -1;
+    *need = r.mode == kDgInside || r.mode == kDgEdge ? dg_need(e, r.reach) : -1;
     return r;
 }
 
@@ -673,12 +673,11 @@ __global__ void __launch_bounds__(kDgThreads, 3)
             reinterpret_cast<float4*>(row)[lane] = ch[h];
             if (lane == 0) row[2 * kDgHalf] = 0.0f;
             __syncwarp();
-            const float two = 2.0f * rec[h].reach;
-            const int m = static_cast<int>(fminf(two, 2.0f * kDgHalf));
-            const float g = two - static_cast<float>(m);
+            const int m = dg_spread(rec[h].reach);
+            const float g = 2.0f * rec[h].reach - static_cast<float>(m);
             // the pieces that the tile's positions can fall in
-            for (int i = kDgHalf - need[h] + lane; i < kDgHalf + need[h]; i += 32) {
-                const float right = row[i + 1], after = row[i - m + 1], before = row[max(i - m, 0)];
+            for (int i = dg_first_piece(need[h], m) + lane; i < kDgHalf + need[h]; i += 32) {
+                const float right = row[i + 1], after = row[i - m + 1], before = row[i - m];
                 float sum = m > 0 ? row[i] : 0.0f;
                 if (m > 1) sum += after;
                 for (int k = i - m + 2; k < i; ++k) sum += row[k];
