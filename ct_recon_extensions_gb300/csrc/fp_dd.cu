@@ -511,7 +511,9 @@ __global__ void __launch_bounds__(kDdThreads)
 // into the next view's row (the staging reads on likewise), and a footprint
 // that starts at or before -1/2 adds nothing (tiles that reach there test it
 // per pixel, in FP64 within 1e-3 of it).  Pixels at the ends of their line have
-// one-sided footprints: dd_grad_border sums those and overwrites them.
+// one-sided footprints: dd_grad_border sums those and overwrites them.  A (tile,
+// view) with an infinity, NaN or a value beyond 1e30 among its pieces is summed
+// pixel by pixel.
 //
 // CTA: 32 x 64 pixels, 8 of one column per thread, a segment of the views in
 // blocks of kDgViews; the next block's channels are loaded into registers
@@ -527,7 +529,7 @@ constexpr float kDgMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an i
 struct DdView {
     long long b, o, l;  // 32.32 fixed point
     float of, lf;       // o and l
-    float half_w;       // half the view's weight
+    float w;            // the view's weight
     int flags;          // kDgUx: lines are rows; kDgBad: not of this form, or out of range
 };
 constexpr int kDgUx = 1, kDgBad = 2;
@@ -548,12 +550,13 @@ __global__ void __launch_bounds__(256)
     ok = __all_sync(0xffffffffu, ok);
     if (lane == 0)
         views[ia] = DdView{ok ? fix32(b) : 0, ok ? fix32(o) : 0, ok ? fix32(l) : 0, static_cast<float>(o),
-                           static_cast<float>(l), 0.5f * static_cast<float>(weights[ia]), (usex[ia] ? kDgUx : 0) | (ok ? 0 : kDgBad)};
+                           static_cast<float>(l), static_cast<float>(weights[ia]), (usex[ia] ? kDgUx : 0) | (ok ? 0 : kDgBad)};
 }
 
 // A pixel-view by itself, for any view: whether it adds anything, its first
 // channel, their count and the footprint's ends relative to the first, from
-// integers (in FP64 within 2^-16 of the row's start, and for views not of
+// integers (in FP64 within 2^-16 of where a channel begins or ends, so that the
+// cells of no length that the reference reads are read, and for views not of
 // DdView's form).
 __device__ __forceinline__ bool dd_grad_one(const DdView& v, const double* __restrict__ pp, int ix, int iy, int n,
                                             long long room, int& first, int& cnt, float& lr, float& rr)
@@ -567,15 +570,29 @@ __device__ __forceinline__ bool dd_grad_one(const DdView& v, const double* __res
         left = right;
         right = t;
     }
-    const long long c = (left + kDdHalf) >> 32;  // the left end's cell
+    const long long L = left + kDdHalf, R = right + kDdHalf;
+    const unsigned lf = static_cast<unsigned>(L), rf = static_cast<unsigned>(R);
+    if ((v.flags & kDgBad) || lf < kDdFxGuard || lf > 0u - kDdFxGuard || rf < kDdFxGuard || rf > 0u - kDdFxGuard)
+        return dd_grad_decide64(pp, ux, ix, iy, n, n, room, first, cnt, lr, rr);
+    const long long c = L >> 32;  // the left end's cell
     first = static_cast<int>(c);
-    cnt = static_cast<int>(((right + kDdHalf) >> 32) - c) + 1;
+    cnt = static_cast<int>((R >> 32) - c) + 1;
     lr = static_cast<float>(left - (c << 32)) * 2.3283064365386963e-10f;
     rr = static_cast<float>(right - (c << 32)) * 2.3283064365386963e-10f;
-    const long long past = left + kDdHalf;  // > 0: the view counts (tie: decided in FP64)
-    if ((v.flags & kDgBad) || (past > -(1ll << 16) && past < (1ll << 16)))
-        return dd_grad_decide64(pp, ux, ix, iy, n, n, room, first, cnt, lr, rr);
-    return past > 0;
+    return c >= 0;
+}
+
+// The term of a pixel-view, less the view's weight.
+__device__ __forceinline__ float dd_grad_term(const float* __restrict__ P, long long row, long long total, int first,
+                                              int cnt, float lr, float rr)
+{
+    float t = 0.0f;
+    for (int c = 0; c < cnt; ++c) {
+        const float fc = static_cast<float>(c);
+        const float len = fminf(fc + 0.5f, rr) - fmaxf(fc - 0.5f, lr);
+        if (row + first + c < total) t = fmaf(len, __ldg(P + row + first + c) * 0.5f, t);
+    }
+    return t;
 }
 
 // A view on a tile.
@@ -656,9 +673,10 @@ __global__ void __launch_bounds__(kDgThreads, 3)
             int kc;
             rec[h] = dg_record(v, tx0, ty0, &kc, &need[h]);
             const long long row = static_cast<long long>(ia) * ns, room = min(total - row, 0x7fffffffll);
+            const float half_w = 0.5f * v.w;
             auto one = [&](int i) {
                 const int rel = 4 * lane + i - kDgHalf, c = kc + rel;
-                return abs(rel) <= need[h] && c >= 0 && c < static_cast<int>(room) ? __ldg(P + row + c) * v.half_w : 0.0f;
+                return abs(rel) <= need[h] && c >= 0 && c < static_cast<int>(room) ? __ldg(P + row + c) * half_w : 0.0f;
             };
             ch[h] = make_float4(one(0), one(1), one(2), one(3));
         }
@@ -675,6 +693,7 @@ __global__ void __launch_bounds__(kDgThreads, 3)
             __syncwarp();
             const int m = dg_spread(rec[h].reach);
             const float g = 2.0f * rec[h].reach - static_cast<float>(m);
+            bool fine = true;
             // the pieces that the tile's positions can fall in
             for (int i = dg_first_piece(need[h], m) + lane; i < kDgHalf + need[h]; i += 32) {
                 const float right = row[i + 1], after = row[i - m + 1], before = row[i - m];
@@ -682,9 +701,13 @@ __global__ void __launch_bounds__(kDgThreads, 3)
                 if (m > 1) sum += after;
                 for (int k = i - m + 2; k < i; ++k) sum += row[k];
                 const float sa = right - before, sb = right - after;
-                s_piece[j][0][i] = make_float2(fmaf(0.5f, sa, fmaf(g, before, sum)), sa);  // from f = 1/2
-                s_piece[j][1][i] = make_float2(fmaf(0.5f, sb, fmaf(g, after, sum)), sb);
+                const float a = fmaf(0.5f, sa, fmaf(g, before, sum)), b = fmaf(0.5f, sb, fmaf(g, after, sum));
+                s_piece[j][0][i] = make_float2(a, sa);  // from f = 1/2
+                s_piece[j][1][i] = make_float2(b, sb);
+                fine = fine && fabsf(a) + fabsf(sa) < 1e30f && fabsf(b) + fabsf(sb) < 1e30f;
             }
+            // an infinity's slope would take its value away again
+            if (!__all_sync(0xffffffffu, fine)) rec[h].mode = kDgSlow;
             if (lane == 0) s_rec[j] = rec[h];
         }
     };
@@ -712,14 +735,10 @@ __global__ void __launch_bounds__(kDgThreads, 3)
                     if (ix < n && iy < n &&
                         dd_grad_one(v, pos + static_cast<size_t>(v0 + j) * n * 2, ix, iy, n, total - 1 - row, first, cnt,
                                     lr, rr))
-                        for (int c = 0; c < cnt; ++c) {
-                            const float fc = static_cast<float>(c);
-                            const float len = fminf(fc + 0.5f, rr) - fmaxf(fc - 0.5f, lr);
-                            if (first + c >= 0 && row + first + c < total) t = fmaf(len, __ldg(P + row + first + c), t);
-                        }
+                        t = dd_grad_term(P, row, total, first, cnt, lr, rr);
 #pragma unroll
                     for (int q = 0; q < kDgRows; ++q)  // blk stays in registers
-                        if (q == k) blk[q] = fmaf(t, v.half_w, blk[q]);
+                        if (q == k) blk[q] = fmaf(t, v.w, blk[q]);
                 }
                 continue;
             }
@@ -795,14 +814,7 @@ __global__ void __launch_bounds__(kDbThreads)
         int first, cnt;
         float lr, rr;
         if (!dd_grad_one(v, pos + static_cast<size_t>(ia) * n * 2, ix, iy, n, total - 1 - row, first, cnt, lr, rr)) continue;
-        float t = 0.0f;
-        for (int k = 0; k < cnt; ++k) {
-            const long long at = row + first + k;
-            const float fk = static_cast<float>(k);
-            const float len = fminf(fk + 0.5f, rr) - fmaxf(fk - 0.5f, lr);
-            if (first + k >= 0 && at < total) t = fmaf(len, __ldg(P + at), t);
-        }
-        sum = fmaf(t, v.half_w, sum);
+        sum = fmaf(dd_grad_term(P, row, total, first, cnt, lr, rr), v.w, sum);
     }
     s_sum[warp][lane] = sum;
     __syncthreads();
