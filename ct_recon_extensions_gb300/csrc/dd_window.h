@@ -20,10 +20,11 @@ CTR_DD_HD bool dg_fits(float e, float reach) { return e + reach < kDgHalf - 3; }
 CTR_DD_HD int dg_need(float e, float reach) { return static_cast<int>(e + reach) + 2; }
 // Whole channels between a footprint's ends: a piece i is formed from the
 // staged channels i - m .. i + 1 (channel 0 is kDgHalf before the centre).
-CTR_DD_HD int dg_spread(float reach)
+// `two`: twice the reach, 32.32 fixed point.
+CTR_DD_HD int dg_spread(long long two)
 {
-    const float two = 2.0f * reach;
-    return static_cast<int>(two < 2.0f * kDgHalf ? two : 2.0f * kDgHalf);
+    const long long m = two >> 32;
+    return static_cast<int>(m < 2 * kDgHalf ? m : 2 * kDgHalf);
 }
 // Pieces are formed from here to kDgHalf + need - 1: the ones before are past
 // no tile's position, and would read in front of the channels.

@@ -505,8 +505,10 @@ __global__ void __launch_bounds__(kDdThreads)
 // j + 1; with m = floor(2 o) and g = 2 o - m, the left end lies in cell j - m
 // where f < g, else in cell j - m + 1, and the integral is
 //   p[j-m+1] + ... + p[j] + g p[left] + f (p[j+1] - p[left]).
-// It is continuous in x, so the position needs no exact decision: it is FP32
-// relative to the window's centre, from the tile's 32.32 fixed-point reference.
+// It is continuous in x, so the position needs no exact decision: it is fixed
+// point at the middle of a thread's 8 rows, and FP32 along them, relative to the
+// channel nearest there (relative to the window's centre, up to 60 channels away,
+// cost digits: 5.5e-7 against 1.8e-7 from FP64 for noise on 64^2).
 // Two things of the reference are decided: channels past the row's end read on
 // into the next view's row (the staging reads on likewise), and a footprint
 // that starts at or before -1/2 adds nothing (tiles that reach there test it
@@ -598,13 +600,16 @@ __device__ __forceinline__ float dd_grad_term(const float* __restrict__ P, long 
 // A view on a tile.
 enum DgMode { kDgSkip, kDgInside, kDgEdge, kDgSlow };
 struct DgRec {
-    float base, sx, sy;  // y - 1/2 of the tile's reference pixel, relative to the window's centre, and its slopes
-    float knot;          // g - 1/2
-    float limit;         // footprints with y - 1/2 at or below it add nothing
+    // y - 1/2 of the tile's first column half a row below its fourth row,
+    // relative to the window's centre, and its steps: 32.32 fixed point
+    long long base, sx, sy;
+    float syf;    // sy
+    float knot;   // g - 1/2
+    float limit;  // footprints with y - 1/2 at or below it add nothing
     int mode;
-    float reach;  // o
-    int flags;    // the view's
+    int m, ux;  // whole channels of a footprint; whether lines are rows
 };
+static_assert(sizeof(DgRec) == 48, "16-byte loads");
 
 __device__ __forceinline__ DgRec dg_record(const DdView& v, int tx0, int ty0, int* centre, int* need)
 {
@@ -614,29 +619,33 @@ __device__ __forceinline__ DgRec dg_record(const DdView& v, int tx0, int ty0, in
     const long long mid = v.b + (ux ? cx : cy) * v.o + (ux ? cy : cx) * v.l;
     const long long kc = (mid + kDdHalf) >> 32;
     DgRec r;
-    r.sx = ux ? v.of : v.lf;
-    r.sy = ux ? v.lf : v.of;
-    r.reach = fabsf(v.of);
-    r.base = static_cast<float>(static_cast<int>(mid)) * 2.3283064365386963e-10f + (r.reach - 1.0f);  // mid - kc
-    r.knot = 2.0f * r.reach - floorf(2.0f * r.reach) - 0.5f;
-    r.flags = v.flags;
+    r.sx = ux ? v.o : v.l;
+    r.sy = ux ? v.l : v.o;
+    r.syf = ux ? v.lf : v.of;
+    const long long o = v.o < 0 ? -v.o : v.o;
+    const float reach = fabsf(v.of);
+    r.base = mid - (kc << 32) + o - (1ll << 32) - kDgTileX / 2 * r.sx - (kDgTileY / 2 - 3) * r.sy + (r.sy >> 1);
+    r.m = dg_spread(2 * o);
+    r.knot = static_cast<float>(static_cast<int>((2 * o - (static_cast<long long>(r.m) << 32)) - kDdHalf)) *
+             2.3283064365386963e-10f;
+    r.ux = ux;
     // positions of the tile lie within e of the centre
-    const float e = fabsf(r.sx) * (kDgTileX / 2) + fabsf(r.sy) * (kDgTileY / 2) + 0.51f;
+    const float e = fabsf(ux ? v.of : v.lf) * (kDgTileX / 2) + fabsf(r.syf) * (kDgTileY / 2) + 0.51f;
     const float start = -0.5f - fmaxf(fminf(static_cast<float>(kc), 1e6f), -1e6f);  // channel -1/2, from the centre
-    r.limit = start + (2.0f * r.reach - 1.0f);
+    r.limit = start + (2.0f * reach - 1.0f);
     // A view whose lines run across its channels (angles outside [0, 2 pi) are
     // not folded) has footprints narrow beside the tile, and a weight to match:
     // positions within the tile in FP32 would cost it digits (5e-5 of the peak
     // against 3e-7).
-    const bool across = fabsf(v.lf) > 2.0f * r.reach;
-    if ((v.flags & kDgBad) || across || !dg_fits(e, r.reach) || kc <= -1000000 || kc >= 0x40000000)
+    const bool across = fabsf(v.lf) > 2.0f * reach;
+    if ((v.flags & kDgBad) || across || !dg_fits(e, reach) || kc <= -1000000 || kc >= 0x40000000)
         r.mode = kDgSlow;
     else if (e < start - 0.01f)
         r.mode = kDgSkip;
     else
-        r.mode = -e - r.reach > start + 0.01f ? kDgInside : kDgEdge;
+        r.mode = -e - reach > start + 0.01f ? kDgInside : kDgEdge;
     *centre = static_cast<int>(kc);
-    *need = r.mode == kDgInside || r.mode == kDgEdge ? dg_need(e, r.reach) : -1;
+    *need = r.mode == kDgInside || r.mode == kDgEdge ? dg_need(e, reach) : -1;
     return r;
 }
 
@@ -648,7 +657,7 @@ __global__ void __launch_bounds__(kDgThreads, 3)
     constexpr unsigned kSecond = 2 * kDgHalf * sizeof(float2);  // from a piece before the knot to the one after it
     __shared__ __align__(16) float2 s_piece[kDgViews][2][2 * kDgHalf];
     __shared__ __align__(16) float s_row[8][2 * kDgHalf + 4];  // a warp's channels while it forms the pieces
-    __shared__ DgRec s_rec[kDgViews];
+    __shared__ __align__(16) DgRec s_rec[2][kDgViews];  // the block's and the next one's
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tx0 = blockIdx.x * kDgTileX, ty0 = blockIdx.y * kDgTileY;
     const int seg = blockIdx.z % segs, b = blockIdx.z / segs;
@@ -656,22 +665,21 @@ __global__ void __launch_bounds__(kDgThreads, 3)
     const long long total = static_cast<long long>(na) * ns;
     const float* P = proj + b * static_cast<size_t>(total);
     const int ix = tx0 + lane, iy0 = ty0 + warp * kDgRows;
-    const float ox = static_cast<float>(lane - kDgTileX / 2), oy = static_cast<float>(warp * kDgRows - kDgTileY / 2);
 
     // staging: a warp takes views warp and warp + 8 of a block, four channels a lane
     constexpr int kPer = kDgViews / 8;
     static_assert(2 * kDgHalf == 4 * 32 && kDgThreads == 256, "four channels a lane, eight warps");
     float4 ch[kPer];
-    DgRec rec[kPer];
     int need[kPer];
-    auto load = [&](int v0) {
+    auto load = [&](int v0, int buf) {
 #pragma unroll
         for (int h = 0; h < kPer; ++h) {
             const int ia = v0 + warp + 8 * h;
             if (ia >= ve) continue;
             const DdView v = views[ia];
             int kc;
-            rec[h] = dg_record(v, tx0, ty0, &kc, &need[h]);
+            const DgRec rec = dg_record(v, tx0, ty0, &kc, &need[h]);
+            if (lane == 0) s_rec[buf][warp + 8 * h] = rec;
             const long long row = static_cast<long long>(ia) * ns, room = min(total - row, 0x7fffffffll);
             const float half_w = 0.5f * v.w;
             auto one = [&](int i) {
@@ -681,7 +689,7 @@ __global__ void __launch_bounds__(kDgThreads, 3)
             ch[h] = make_float4(one(0), one(1), one(2), one(3));
         }
     };
-    auto stage = [&](int v0) {
+    auto stage = [&](int v0, int buf) {
 #pragma unroll
         for (int h = 0; h < kPer; ++h) {
             const int j = warp + 8 * h;
@@ -691,8 +699,8 @@ __global__ void __launch_bounds__(kDgThreads, 3)
             reinterpret_cast<float4*>(row)[lane] = ch[h];
             if (lane == 0) row[2 * kDgHalf] = 0.0f;
             __syncwarp();
-            const int m = dg_spread(rec[h].reach);
-            const float g = 2.0f * rec[h].reach - static_cast<float>(m);
+            const int m = s_rec[buf][j].m;
+            const float g = s_rec[buf][j].knot + 0.5f;
             bool fine = true;
             // the pieces that the tile's positions can fall in
             for (int i = dg_first_piece(need[h], m) + lane; i < kDgHalf + need[h]; i += 32) {
@@ -707,23 +715,23 @@ __global__ void __launch_bounds__(kDgThreads, 3)
                 fine = fine && fabsf(a) + fabsf(sa) < 1e30f && fabsf(b) + fabsf(sb) < 1e30f;
             }
             // an infinity's slope would take its value away again
-            if (!__all_sync(0xffffffffu, fine)) rec[h].mode = kDgSlow;
-            if (lane == 0) s_rec[j] = rec[h];
+            if (!__all_sync(0xffffffffu, fine) && lane == 0) s_rec[buf][j].mode = kDgSlow;
         }
     };
 
     const unsigned pieces = static_cast<unsigned>(__cvta_generic_to_shared(&s_piece[0][0][kDgHalf])) -
                             (__float_as_uint(kDgMagic) << 3);
     float acc[kDgRows] = {};
-    load(vb);
-    for (int v0 = vb; v0 < ve; v0 += kDgViews) {
+    load(vb, 0);
+    int buf = 0;
+    for (int v0 = vb; v0 < ve; v0 += kDgViews, buf ^= 1) {
         const int nv = min(kDgViews, ve - v0);
-        stage(v0);
+        stage(v0, buf);
         __syncthreads();
-        load(v0 + kDgViews);
+        load(v0 + kDgViews, buf ^ 1);
         float blk[kDgRows] = {};  // this block's sums
         for (int j = 0; j < nv; ++j) {
-            const DgRec r = s_rec[j];
+            const DgRec r = s_rec[buf][j];
             if (r.mode == kDgSkip) continue;
             if (r.mode == kDgSlow) {
                 const long long row = static_cast<long long>(v0 + j) * ns;
@@ -742,13 +750,17 @@ __global__ void __launch_bounds__(kDgThreads, 3)
                 }
                 continue;
             }
-            const unsigned at = pieces + j * static_cast<unsigned>(sizeof s_piece[0]), at2 = at + kSecond;
-            const float xc = fmaf(ox, r.sx, r.base);
-            const float2 sy = make_float2(r.sy, r.sy), x0 = make_float2(xc, xc);
+            // the thread's column between its fourth and fifth row: the nearest
+            // channel, and the way past it, so that FP32 holds its rows' positions
+            const long long X = r.base + lane * r.sx + warp * kDgRows * r.sy;
+            const int J = static_cast<int>((X + kDdHalf) >> 32);
+            const float xf = static_cast<float>(static_cast<int>(X)) * 2.3283064365386963e-10f;
+            const unsigned at = pieces + j * static_cast<unsigned>(sizeof s_piece[0]) + 8 * J, at2 = at + kSecond;
+            const float2 sy = make_float2(r.syf, r.syf), x0 = make_float2(xf, xf);
             auto rows = [&](auto keep) {
 #pragma unroll
                 for (int k = 0; k < kDgRows; k += 2) {
-                    const float2 y = __ffma2_rn(make_float2(oy + k, oy + (k + 1)), sy, x0);
+                    const float2 y = __ffma2_rn(make_float2(k - 3.5f, k - 2.5f), sy, x0);
                     const float2 t = __fadd2_rn(y, make_float2(kDgMagic, kDgMagic));
                     const float2 f = __ffma2_rn(__fadd2_rn(t, make_float2(-kDgMagic, -kDgMagic)),
                                                 make_float2(-1.0f, -1.0f), y);
@@ -765,16 +777,17 @@ __global__ void __launch_bounds__(kDgThreads, 3)
             if (r.mode == kDgInside) {
                 rows([](float2, int, float2&, float2&) {});
             } else {  // footprints that start before the first channel are left out
+                const float limit = r.limit - static_cast<float>(J);
                 rows([&](float2 y, int k, float2& p, float2& q) {
                     auto on = [&](float yk, int iy) {
-                        if (fabsf(yk - r.limit) < 1e-3f && ix < n && iy < n) {
+                        if (fabsf(yk - limit) < 1e-3f && ix < n && iy < n) {
                             int first, cnt;
                             float lr, rr;
-                            return dd_grad_decide64(pos + static_cast<size_t>(v0 + j) * n * 2, r.flags & kDgUx, ix, iy,
+                            return dd_grad_decide64(pos + static_cast<size_t>(v0 + j) * n * 2, r.ux, ix, iy,
                                                     n, n, total - 1 - static_cast<long long>(v0 + j) * ns, first, cnt,
                                                     lr, rr);
                         }
-                        return yk > r.limit;
+                        return yk > limit;
                     };
                     if (!on(y.x, iy0 + k)) p = make_float2(0.0f, 0.0f);
                     if (!on(y.y, iy0 + k + 1)) q = make_float2(0.0f, 0.0f);

@@ -17,7 +17,7 @@ int main()
             const float reach = re / 16.0f, e = 0.51f + ex / 16.0f;
             if (!dg_fits(e, reach)) continue;
             ++cases;
-            const int need = dg_need(e, reach), m = dg_spread(reach);
+            const int need = dg_need(e, reach), m = dg_spread(static_cast<long long>(2.0 * reach * 4294967296.0));
             const int first = dg_first_piece(need, m), end = kDgHalf + need;
             bool ok = first - m >= 0 && end <= 2 * kDgHalf;  // reads [first - m, end], one zero behind the channels
             // positions y = x + reach - 1 with |x| <= e round to pieces; a hair more for the FP32 positions
