@@ -140,7 +140,9 @@ __global__ void __launch_bounds__(kDdThreads)
 // A footprint's width is the same on every line, and up to two pixels (every
 // view when ds <= sqrt(2) dx) it covers at most three intervals: all lines but
 // those at the image's edges run a loop without an interval count or a
-// division, the common width divided out at the end.  One lane per ray, a
+// division, its sums scaled by the common width's reciprocal four lines at a time
+// (one sum over all lines cost digits: noise on 512^2 5.3e-7 from FP64, now 2.2e-7,
+// 3.8e-7 line by line with a division each).  One lane per ray, a
 // block's lanes on adjacent channels of one view, the warp's rays on the same
 // line, so that each load reads adjacent pixels.  Blocks follow one another by
 // view, chunk of channels by chunk: neighbouring views' rays through the same
@@ -246,7 +248,8 @@ __global__ void __launch_bounds__(kDdRayThreads, 14)
     const bool wide = __any_sync(0xffffffffu, any && !(width >= 0.001f && width <= 2.0f));
     const float ends = sum;
     const long long start = xl;
-    float acc = 0.0f;  // in units of half the width
+    float part;  // a group of lines, in units of half the width
+    const float beyond = width - 1.0f, inv = any ? 0.5f / width : 0.0f;
     // A line's four pixels are loaded whether its footprint reaches them or not
     // (the copies have three zeros behind each line), and get the weight 0 where
     // it does not: a ray that an infinity or NaN reached this way is summed
@@ -254,11 +257,12 @@ __global__ void __launch_bounds__(kDdRayThreads, 14)
     auto step = [&](const float* __restrict__ line) {
         const float* p = line + static_cast<int>(xl >> 32);
         const float p0 = __ldg(p), p1 = __ldg(p + 1), p2 = __ldg(p + 2), p3 = __ldg(p + 3);
-        const float a = __uint_as_float(0x3F800000u | (static_cast<unsigned>(xl) >> 9));  // 1 + the start's fraction
-        const float e = a + width;
-        acc = fmaf(fminf(e, 2.0f) - a, p0 + p1, acc);
-        acc = fmaf(__saturatef(e - 2.0f), p1 + p2, acc);
-        acc = fmaf(__saturatef(e - 3.0f), p2 + p3, acc);
+        // what is left of the start's interval: exact, so that the three lengths
+        // add up to the width to its own digits, however narrow
+        const float d = 2.0f - __uint_as_float(0x3F800000u | (static_cast<unsigned>(xl) >> 9));
+        part = fmaf(fminf(width, d), p0 + p1, part);
+        part = fmaf(__saturatef(width - d), p1 + p2, part);
+        part = fmaf(__saturatef(beyond - d), p2 + p3, part);
         xl += S;
     };
     // the same for a line that some of the warp's rays may not have, and where
@@ -290,8 +294,10 @@ __global__ void __launch_bounds__(kDdRayThreads, 14)
     } else {
         for (int l = lo; l <= hi; l += kDdUnroll, line += kDdUnroll * w) {
             if (l >= in && l + kDdUnroll - 1 <= out && !__any_sync(0xffffffffu, xl > last || xl + ahead > last)) {
+                part = 0.0f;
 #pragma unroll
                 for (int u = 0; u < kDdUnroll; ++u) step(line + u * w);
+                sum = fmaf(part, inv, sum);
             } else {  // lines past the last one read the last one
 #pragma unroll
                 for (int u = 0; u < kDdUnroll; ++u) step_edge(l + u <= hi ? line + u * w : line, l + u);
@@ -300,13 +306,10 @@ __global__ void __launch_bounds__(kDdRayThreads, 14)
     }
     if (is < ns) {
         const float length = static_cast<float>(ux ? fabs(dy / sincos[2 * ia + 1]) : fabs(dx / sincos[2 * ia]));
-        if (any && !wide) {
-            sum += acc * (0.5f / width);
-            if (!isfinite(sum)) {
-                sum = ends;
-                xl = start;
-                for (int l = k0; l <= k1; ++l, xl += S) sum += dd_line(I + l * w, xl, xl + span, n);
-            }
+        if (any && !wide && !isfinite(sum)) {
+            sum = ends;
+            xl = start;
+            for (int l = k0; l <= k1; ++l, xl += S) sum += dd_line(I + l * w, xl, xl + span, n);
         }
         proj[blockIdx.y * proj_stride + ray] = sum * length;
     }
