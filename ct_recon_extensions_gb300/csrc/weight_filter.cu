@@ -403,58 +403,68 @@ __device__ __forceinline__ void filter_rows(const T* __restrict__ in, const doub
 }
 
 // ---- FP32, four rows at a time ------------------------------------------------
-// filter_rows' sums for four rows as packed pairs and eight outputs of a parity
+// filter_rows' sums for four rows as packed pairs and four outputs of a parity
 // per thread.  The rows lie interleaved in shared memory, so an input of all
 // four is one 16-byte load, and every tap is stored twice, so that it loads as
 // the pair that multiplies two rows: a step is 2 loads, 2 packed differences and
-// 16 packed multiply-adds for 32 products, where filter_span took 4 loads, 3
-// differences and 12 multiply-adds for 12 (its loads bound it, and with four
-// outputs still did).  The inputs are split over groups of threads, whose sums
-// are added in order.  One CTA alone takes 14 us at 729 channels: 3.5 staging
-// (the taps come in FP64, whose unit is slow), 9 the sums, at half of the FP32
-// rate.  16 x 1000 x 700: 391 -> 208 us; 720 x 729: 23.5 -> 20.2.
-constexpr int kQuadRows = 4, kQuadOut = 8;
-constexpr size_t kQuadSmemMax = 216 * 1024;
-constexpr int kQuadMany = 192;  // task threads of a CTA in launches of many CTAs
+// 8 packed multiply-adds for 16 products, where filter_span took 4 loads, 3
+// differences and 12 multiply-adds for 12 (its loads bound it).  The inputs are
+// split over groups of threads, whose sums are added in order; how, depends on
+// the channels alone, so that a row's result does not on the rows beside it.
+// Bound by the packed FP32 unit, 10 operations a step.  720 x 729: 24.3 -> 23.7
+// us; 4 x 720 x 729: 84 -> 52; 16 x 1000 x 700: 392 -> 248; 2304 x 1472: 238 -> 147;
+// 1472 x 2304: 381 -> 285.  Eight outputs a thread with one reference value took
+// 20.9, 48, 207, 149 and 333, and cost digits (phantoms on 500 channels 5.9e-7 from
+// FP64 in filter_rows, 9.3e-7 so, here 4.5e-7); with two reference values they
+// spill (255 us for the third).
+constexpr int kQuadRows = 4, kQuadOut = 4;
+constexpr size_t kQuadSmemMax = 226 * 1024;
+constexpr int kQuadThreads = 384;  // task threads of a CTA, two CTAs an SM
+constexpr int kQuadWide = 992;     // those of rows with more tasks, where they fit
 // Tap idx lies at pair 10 (idx / 8) + idx % 8: the 16 lanes of a half-warp's
-// load (taps 16 q + p, q < 8, p < 2) fall in distinct banks but for one pair.
+// load (taps 8 q + p, q < 8, p < 2) fall in distinct banks.
 constexpr int kQuadGroup = 10;
 __host__ __device__ inline int quad_slot(int idx) { return kQuadGroup * (idx >> 3) + (idx & 7); }
 __host__ __device__ inline int quad_taps(unsigned ns) { return quad_slot(2 * static_cast<int>(ns) + 2 * kFilterPad + 8); }
-// Tasks (16-output block, parity) of a row and the parts that their inputs are
-// split into, each rounded up to whole warps; one more warp forms C and the tail
-// sums.
-__host__ __device__ inline int quad_tasks(unsigned ns) { return static_cast<int>((ns + 15) / 16) * 2; }
-__host__ __device__ inline int quad_stride(unsigned ns) { return (quad_tasks(ns) + 31) / 32 * 32; }
-__host__ __device__ inline int quad_parts(unsigned ns, int threads)
+// Tasks (filter_tasks: 8-output block, parity) of a row and the parts that their
+// inputs are split into, each rounded up to whole warps; one more warp forms C and
+// the tail sums.
+__host__ __device__ inline int quad_stride(unsigned ns) { return (filter_tasks(ns) + 31) / 32 * 32; }
+__host__ __device__ inline int quad_parts(unsigned ns)
 {
-    const int p = threads / quad_stride(ns);
+    const int p = kQuadThreads / quad_stride(ns);
     return p < 1 ? 1 : (p > 8 ? 8 : p);
 }
 inline int quad_block(unsigned ns, int threads)
 {
     const int t = quad_stride(ns);
-    return (t > threads ? threads : t * quad_parts(ns, threads)) + 32;
+    return (t > threads ? threads : t * quad_parts(ns)) + 32;
 }
-// Shared layout: inputs [ns] of four rows, the later parts' sums [part][output][task]
-// (at most one value a thread), taps, tail sums.
-inline size_t quad_smem(unsigned ns, int threads)
+// A thread's sums are put by in shared memory at least every kQuadFold inputs
+// (blocked summation), where there is room for it: 1472 channels 2.0e-6 from FP64
+// in one sum of 736, 7.9e-7 in two halves, 4.7e-7 so.
+constexpr int kQuadFold = 128;
+constexpr unsigned kFilterBatchMaxNs = 4904;  // of a batched launch
+// Threads that take tasks: the extra warp too, once the tasks are more than a CTA's.
+inline int quad_slots(unsigned ns, int nthr) { return filter_tasks(ns) > nthr ? nthr + 32 : nthr; }
+// Shared layout: inputs [ns] of four rows, the threads' sums [output][slot], taps,
+// tail sums.
+inline size_t quad_smem(unsigned ns, int slots)
 {
-    return sizeof(float4) * ns + sizeof(float4) * kQuadOut * threads + sizeof(float2) * quad_taps(ns) +
-           filter_tail_bytes(ns);
+    return sizeof(float4) * (ns + kQuadOut * slots) + sizeof(float2) * quad_taps(ns) + filter_tail_bytes(ns);
 }
 
 __device__ __forceinline__ float2 pair_of(float v) { return make_float2(v, v); }
 
-// Inputs j0, j0 + 2, ... < j1 into the outputs i0 + 2 m: acc[m][0] rows 0 and 1,
-// acc[m][1] rows 2 and 3.
+// Inputs j0, j0 + 2, ... < j1, less the reference values c, into the outputs
+// i0 + 2 m: acc[m][0] rows 0 and 1, acc[m][1] rows 2 and 3.
 __device__ __forceinline__ void quad_span(const float4* __restrict__ xs, int j0, int j1, int i0, int d0,
-                                          const float2* __restrict__ Hd, float2 ca, float2 cb,
+                                          const float2* __restrict__ Hd, const float4& c,
                                           float2 (&acc)[kQuadOut][2])
 {
     const float2 minus = pair_of(-1.0f);
     int idx = i0 - j0 + d0;  // the tap of output i0 and input j
-    float2 w[kQuadOut];      // tap of output m at w[(m + turn) % 8]
+    float2 w[kQuadOut];      // tap of output m at w[(m - turn) % 4]
 #pragma unroll
     for (int m = 0; m < kQuadOut; ++m) w[m] = Hd[quad_slot(idx + 2 * m)];
     // eight inputs move the taps by two groups: the same places twenty pairs back
@@ -463,18 +473,19 @@ __device__ __forceinline__ void quad_span(const float4* __restrict__ xs, int j0,
     for (int k = 0; k < 4; ++k) h[k] = Hd + quad_slot(idx - 2 - 2 * k);
     int j = j0;
     auto step = [&](float4 x, int turn) {
-        const float2 xa = __ffma2_rn(ca, minus, make_float2(x.x, x.y)), xb = __ffma2_rn(cb, minus, make_float2(x.z, x.w));
+        const float2 xa = __ffma2_rn(make_float2(c.x, c.y), minus, make_float2(x.x, x.y));
+        const float2 xb = __ffma2_rn(make_float2(c.z, c.w), minus, make_float2(x.z, x.w));
 #pragma unroll
         for (int m = 0; m < kQuadOut; ++m) {
-            acc[m][0] = __ffma2_rn(w[(m + kQuadOut - turn) % kQuadOut], xa, acc[m][0]);
-            acc[m][1] = __ffma2_rn(w[(m + kQuadOut - turn) % kQuadOut], xb, acc[m][1]);
+            acc[m][0] = __ffma2_rn(w[(m + 2 * kQuadOut - turn) % kQuadOut], xa, acc[m][0]);
+            acc[m][1] = __ffma2_rn(w[(m + 2 * kQuadOut - turn) % kQuadOut], xb, acc[m][1]);
         }
     };
     for (; j + 14 < j1; j += 16) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             step(xs[j + 2 * k], k);
-            w[7 - k] = h[k & 3][k < 4 ? 0 : -kQuadGroup];  // the new tap takes the place of output 7's
+            w[(7 - k) % kQuadOut] = h[k & 3][k < 4 ? 0 : -kQuadGroup];  // the new tap takes the place of the last output's
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) h[k] -= 2 * kQuadGroup;
@@ -492,21 +503,22 @@ __device__ __forceinline__ void quad_span(const float4* __restrict__ xs, int j0,
 template <bool kGrad>
 __device__ __forceinline__ void filter_quad(const float* __restrict__ in, const double* __restrict__ filter,
                                             float* __restrict__ out, const float* __restrict__ weight, unsigned ns,
-                                            unsigned long long r0, int nr, double ds, int parts,
+                                            unsigned long long r0, int nr, double ds, int slots,
                                             unsigned char* smem_raw)
 {
     const int n = static_cast<int>(ns), nodd = n / 2;  // odd offsets in [1, n-1]
-    const int tasks = quad_tasks(ns);
+    const int tasks = filter_tasks(ns);
     float4* xs = reinterpret_cast<float4*>(smem_raw);
-    float4* red = xs + n;  // [part - 1][output][task]
-    float2* Hd = reinterpret_cast<float2*>(red + static_cast<size_t>(kQuadOut) * tasks * (parts - 1));
+    const int nthr = static_cast<int>(blockDim.x) - 32;  // the task threads; one more warp forms C and the tail sums
+    const int parts = quad_parts(ns);
+    float4* red = xs + n;  // [output][thread]
+    float2* Hd = reinterpret_cast<float2*>(red + kQuadOut * slots);
     float* Pt = reinterpret_cast<float*>(Hd + quad_taps(ns));
     float* Qt = Pt + nodd + 2;
     float* Cs = Qt + nodd + 2;
     const int d0 = (n - 1) + kFilterPad;
     auto H = [&](int d) { return Hd[quad_slot(d + d0)].x; };
     __shared__ int s_even;
-    const int nthr = static_cast<int>(blockDim.x) - 32;  // the task threads; one more warp forms C and the tail sums
 
     const double* h = filter + ns;  // h[k], k in [-ns, ns]
     if (threadIdx.x == 0) s_even = 0;
@@ -568,8 +580,31 @@ __device__ __forceinline__ void filter_quad(const float* __restrict__ in, const 
         if (lane == 0) Cs[0] = static_cast<float>((h[0] + cs) * ds);
     }
     if (parts == 1) __syncthreads();  // the tasks write outputs as they go: the sums first
+    // the reference value of a task's rows: the input next to its outputs
+    auto refs = [&](int i0) { return xs[min(i0 + 3, n - 1)]; };
+    // this thread's sums over the inputs ja, ja + 2, ... < je, at most kQuadFold at a
+    // time, the earlier ones' total in `red`
+    auto sums = [&](int ja, int je, int i0, const float4& c, float2 (&acc)[kQuadOut][2]) {
+        const int cnt = (je - ja + 1) / 2, folds = slots > 0 ? max(1, (cnt + kQuadFold - 1) / kQuadFold) : 1;
+        float4* own = red + threadIdx.x;
+        for (int k = 0; k < folds; ++k) {
+#pragma unroll
+            for (int m = 0; m < kQuadOut; ++m) acc[m][0] = acc[m][1] = make_float2(0.0f, 0.0f);
+            quad_span(xs, ja + 2 * (cnt * k / folds), k + 1 == folds ? je : ja + 2 * (cnt * (k + 1) / folds), i0, d0, Hd, c, acc);
+            if (folds == 1) return;
+#pragma unroll
+            for (int m = 0; m < kQuadOut; ++m) {
+                if (k > 0) {
+                    const float4 v = own[m * slots];
+                    acc[m][0] = __fadd2_rn(acc[m][0], make_float2(v.x, v.y));
+                    acc[m][1] = __fadd2_rn(acc[m][1], make_float2(v.z, v.w));
+                }
+                if (k + 1 < folds) own[m * slots] = make_float4(acc[m][0].x, acc[m][0].y, acc[m][1].x, acc[m][1].y);
+            }
+        }
+    };
     // outputs i0, i0 + 2, ... of a task
-    auto finish = [&](int i0, float4 c, const float2 (&acc)[kQuadOut][2]) {
+    auto finish = [&](int i0, const float4& c, const float2 (&acc)[kQuadOut][2]) {
         const float h0 = H(0);
 #pragma unroll
         for (int m = 0; m < kQuadOut; ++m) {
@@ -587,28 +622,26 @@ __device__ __forceinline__ void filter_quad(const float* __restrict__ in, const 
     if (!s_even && parts > 1) {
         const int stride = quad_stride(ns), part = threadIdx.x / stride, g = threadIdx.x - part * stride;
         const bool active = part < parts && g < tasks;
-        const int i0 = (g >> 1) * 16 + (g & 1);
+        const int i0 = (g >> 1) * 8 + (g & 1);
         float2 acc[kQuadOut][2] = {};
         float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (active) {
-            c = xs[min(i0 + 7, n - 1)];
+            c = refs(i0);
             const int jb = (i0 + 1) & 1;  // inputs of the other parity
             const int cnt = (n - jb + 1) / 2;
-            const int ja = jb + 2 * (cnt * part / parts), je = part + 1 == parts ? n : jb + 2 * (cnt * (part + 1) / parts);
-            quad_span(xs, ja, je, i0, d0, Hd, make_float2(c.x, c.y), make_float2(c.z, c.w), acc);
+            sums(jb + 2 * (cnt * part / parts), part + 1 == parts ? n : jb + 2 * (cnt * (part + 1) / parts), i0, c, acc);
             if (part > 0) {
 #pragma unroll
                 for (int m = 0; m < kQuadOut; ++m)
-                    red[((part - 1) * kQuadOut + m) * tasks + g] =
-                        make_float4(acc[m][0].x, acc[m][0].y, acc[m][1].x, acc[m][1].y);
+                    red[m * slots + threadIdx.x] = make_float4(acc[m][0].x, acc[m][0].y, acc[m][1].x, acc[m][1].y);
             }
         }
         __syncthreads();
         if (active && part == 0) {
-            for (int k = 0; k < parts - 1; ++k)
+            for (int k = 1; k < parts; ++k)
 #pragma unroll
                 for (int m = 0; m < kQuadOut; ++m) {
-                    const float4 v = red[(k * kQuadOut + m) * tasks + g];
+                    const float4 v = red[m * slots + k * stride + g];
                     acc[m][0] = __fadd2_rn(acc[m][0], make_float2(v.x, v.y));
                     acc[m][1] = __fadd2_rn(acc[m][1], make_float2(v.z, v.w));
                 }
@@ -616,10 +649,10 @@ __device__ __forceinline__ void filter_quad(const float* __restrict__ in, const 
         }
     } else if (!s_even) {
         for (int task = threadIdx.x; task < tasks; task += blockDim.x) {
-            const int i0 = (task >> 1) * 16 + (task & 1);
-            float2 acc[kQuadOut][2] = {};
-            const float4 c = xs[min(i0 + 7, n - 1)];
-            quad_span(xs, (i0 + 1) & 1, n, i0, d0, Hd, make_float2(c.x, c.y), make_float2(c.z, c.w), acc);
+            const int i0 = (task >> 1) * 8 + (task & 1);
+            float2 acc[kQuadOut][2];
+            const float4 c = refs(i0);
+            sums((i0 + 1) & 1, n, i0, c, acc);
             finish(i0, c, acc);
         }
     } else {
@@ -643,13 +676,13 @@ __device__ __forceinline__ void filter_quad(const float* __restrict__ in, const 
 template <bool kGrad, int kThreads, int kCtas>
 __global__ void __launch_bounds__(kThreads + 32, kCtas)
     ramp_filter_quad(const float* __restrict__ in, const double* __restrict__ filter, float* __restrict__ out,
-                     const float* __restrict__ weight, unsigned ns, unsigned long long rows, double ds, int parts)
+                     const float* __restrict__ weight, unsigned ns, unsigned long long rows, double ds, int slots)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     grid_dep_wait();  // launched as a dependent of the kernel before it
     // rows dealt evenly over the grid, at most kQuadRows a CTA
     const unsigned long long r0 = blockIdx.x * rows / gridDim.x, r1 = (blockIdx.x + 1ull) * rows / gridDim.x;
-    filter_quad<kGrad>(in, filter, out, weight, ns, r0, static_cast<int>(r1 - r0), ds, parts, smem_raw);
+    filter_quad<kGrad>(in, filter, out, weight, ns, r0, static_cast<int>(r1 - r0), ds, slots, smem_raw);
 }
 
 // False (nothing launched) where a row does not fit the shared memory.
@@ -657,7 +690,10 @@ template <bool kGrad, int kThreads, int kCtas>
 bool launch_quad(const ctr_filter_param* p, const float* in, const double* filter, float* out, const float* weight,
                  unsigned long long rows, cudaStream_t stream, cudaError_t* e)
 {
-    const size_t smem = quad_smem(p->ns, kThreads);
+    const int block = quad_block(p->ns, kThreads);
+    int slots = quad_slots(p->ns, block - 32);
+    if (kThreads == kQuadWide && quad_smem(p->ns, slots) > kQuadSmemMax) slots = 0;  // one sum a thread
+    const size_t smem = quad_smem(p->ns, slots);
     const unsigned long long blocks = (rows + kQuadRows - 1) / kQuadRows;
     auto kern = ramp_filter_quad<kGrad, kThreads, kCtas>;
     if (smem > kQuadSmemMax || blocks > 0x7fffffffull ||
@@ -665,8 +701,8 @@ bool launch_quad(const ctr_filter_param* p, const float* in, const double* filte
         cudaGetLastError();
         return false;
     }
-    *e = launch_dependent(kern, dim3(static_cast<unsigned>(blocks)), dim3(quad_block(p->ns, kThreads)), smem, stream, in,
-                          filter, out, weight, p->ns, rows, p->ds, quad_parts(p->ns, kThreads));
+    *e = launch_dependent(kern, dim3(static_cast<unsigned>(blocks)), dim3(block), smem, stream, in,
+                          filter, out, weight, p->ns, rows, p->ds, slots);
     return true;
 }
 
@@ -693,15 +729,15 @@ __global__ void __launch_bounds__(kFilterMaxThreads)
 }
 
 // Batched FP32 filtering with pre-weighting: one CTA per (job, row block).
-__global__ void __launch_bounds__(kQuadMany + 32, 3)
-    ramp_filter_batch_kernel(const FilterJob* __restrict__ jobs, const int2* __restrict__ blocks)
+__global__ void __launch_bounds__(kQuadThreads + 32, 2)
+    ramp_filter_batch_kernel(const FilterJob* __restrict__ jobs, const int2* __restrict__ blocks, int slots)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int2 b = blocks[blockIdx.x];  // (job, first row)
     const FilterJob J = jobs[b.x];
     const int nr = min(kFilterRowsPerBlock, static_cast<int>(J.nrow) - b.y);
     static_assert(kFilterRowsPerBlock == kQuadRows, "a block's rows");
-    filter_quad<false>(J.in, J.taps, J.out, J.weight, J.ns, b.y, nr, J.ds, quad_parts(J.ns, kQuadMany), smem_raw);
+    filter_quad<false>(J.in, J.taps, J.out, J.weight, J.ns, b.y, nr, J.ds, slots, smem_raw);
 }
 
 template <typename T, bool kGrad>
@@ -717,13 +753,9 @@ int launch_ramp_filter(const ctr_filter_param* p, const T* in, const double* fil
     const unsigned long long rows = static_cast<unsigned long long>(p->nrow) * batch;
     const int threads = filter_block<T>(p->ns);
     if constexpr (sizeof(T) == 4) {
-        const unsigned long long groups = (rows + kQuadRows - 1) / kQuadRows;
         cudaError_t e = cudaSuccess;
-        // Up to two CTAs an SM, more threads on a row; beyond, more CTAs an SM.
-        // 720 x 729: 20.2 against 23.9 us; 4 x 720 x 729: 51.8 against 48.1;
-        // 16 x 1000 x 700: 266 against 208.
-        if (groups <= 2ull * device_sms() ? launch_quad<kGrad, 288, 2>(p, in, filter, out, weight, rows, stream, &e)
-                                          : launch_quad<kGrad, kQuadMany, 3>(p, in, filter, out, weight, rows, stream, &e)) {
+        if (quad_stride(p->ns) > kQuadThreads ? launch_quad<kGrad, kQuadWide, 1>(p, in, filter, out, weight, rows, stream, &e)
+                                              : launch_quad<kGrad, kQuadThreads, 2>(p, in, filter, out, weight, rows, stream, &e)) {
             if (e != cudaSuccess) return fail(CTR_ERR_CUDA, "ramp_filter: %s", cudaGetErrorString(e));
             return check_launch("ramp_filter");
         }
@@ -780,12 +812,13 @@ int ramp_filter_weighted_f32(const ctr_filter_param* p, const float* in, const d
 int ramp_filter_batch_f32(const FilterJob* jobs, const int2* blocks, int n_blocks, unsigned max_ns,
                           cudaStream_t stream)
 {
-    const size_t smem = quad_smem(max_ns, kQuadMany);
-    if (smem > kQuadSmemMax) return fail(CTR_ERR_UNSUPPORTED, "ns=%u too wide for the filter tile", max_ns);
+    const int slots = quad_slots(max_ns, kQuadThreads);
+    const size_t smem = quad_smem(max_ns, slots);
+    if (max_ns > kFilterBatchMaxNs) return fail(CTR_ERR_UNSUPPORTED, "ns=%u too wide for the filter tile", max_ns);
     cudaError_t e = cudaFuncSetAttribute(ramp_filter_batch_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return fail(CTR_ERR_CUDA, "filter smem: %s", cudaGetErrorString(e));
-    if (n_blocks > 0) ramp_filter_batch_kernel<<<n_blocks, kQuadMany + 32, smem, stream>>>(jobs, blocks);
+    if (n_blocks > 0) ramp_filter_batch_kernel<<<n_blocks, kQuadThreads + 32, smem, stream>>>(jobs, blocks, slots);
     return check_launch("ramp_filter_batch");
 }
 

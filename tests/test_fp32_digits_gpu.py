@@ -42,3 +42,43 @@ def test_disdriven_narrow_channels(ds, start):
     op = tc.ParallelProjection2DOp(ns, na, ds, 2 * math.pi / na, 0.25, start, n, n, 1.0, 1.0, 0.3, -0.2, method="disdriven")
     for img in (np.ones((n, n)), np.random.default_rng(2).random((n, n))):
         assert _off(op.forward, img.astype(np.float32)) <= 4e-7
+
+
+def _ramp(ns, nrow, kind="fan"):
+    from ct_recon_extensions_gb300 import torch_ctrecon as tc
+    return tc.RampFilterOp(ns, nrow, 1.3, 900.0 if kind == "fan" else -1.0, 1 if kind == "fan" else 0)
+
+
+@pytest.mark.parametrize("ns", [95, 500, 729, 1472, 1537, 2304, 4100])
+def test_ramp_phantom(ns):
+    """Sinograms of discs: centred sums (the reference input within 8 channels of
+    its outputs) of 128 inputs at most, then of these: partial sums about as large
+    as the result, sqrt(128 + 16) roundings of 2^-24 = 7e-7 at most.  A reference
+    input per 16 outputs gives 9e-7 at 500 channels, sums of 736 inputs 2e-6 at 1472."""
+    rng = np.random.default_rng(ns)
+    s = np.linspace(-1, 1, ns)[None]
+    th = np.linspace(0, math.pi, 48, endpoint=False)[:, None]
+    x = 0.01 * rng.standard_normal((48, ns))
+    for _ in range(10):
+        a, q = rng.uniform(0.05, 0.5), s - rng.uniform(-0.5, 0.5) * np.cos(th + rng.uniform(0, 6))
+        x = x + 4 * np.sqrt(np.clip(a * a - q * q, 0, None))
+    assert _off(_ramp(ns, 48, "par").forward, x.astype(np.float32)) <= 7e-7
+
+
+@pytest.mark.parametrize("ns", [5, 96, 185, 729, 1100, 1600, 4096, 4136, 4137, 4700, 5775, 5800])
+def test_ramp_same_in_any_batch(ns):
+    """A sinogram's result does not depend on those beside it, on either side of
+    two CTAs an SM, forward and grad; wide rows against FP64 within 1e-5."""
+    import torch
+    op = _ramp(ns, 33, "par")
+    x = torch.as_tensor(np.random.default_rng(ns).standard_normal((90, 33, ns)).astype(np.float32), device="cuda")
+    for f in (op.forward, op.adjoint):
+        many = f(x)
+        for i in (0, 41, 89):
+            assert torch.equal(f(x[i]), many[i])
+        if ns > 4000:
+            h = np.array([op.taps(x.device).cpu().numpy()]).ravel()
+            k = np.arange(ns)
+            m = h[ns + k[:, None] - k[None, :]] if f == op.forward else h[ns + k[None, :] - k[:, None]]
+            want = 1.3 * (m @ host(x[41]).astype(np.float64).T).T
+            assert rel_l2(host(many[41]), want) <= 1e-5
