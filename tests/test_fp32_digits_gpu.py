@@ -82,3 +82,17 @@ def test_ramp_same_in_any_batch(ns):
             m = h[ns + k[:, None] - k[None, :]] if f == op.forward else h[ns + k[None, :] - k[:, None]]
             want = 1.3 * (m @ host(x[41]).astype(np.float64).T).T
             assert rel_l2(host(many[41]), want) <= 1e-5
+
+
+@pytest.mark.parametrize("step", [0.05, 0.125, 0.25, 0.5])
+@pytest.mark.parametrize("start", [0.0, 0.013])
+def test_ray_casting(step, start):
+    """Constant images come out to the last rounding or two (a row's weights add up
+    to its samples); discs within the positions' 2^-23 of a pixel at their edges and
+    sums of 8 rows, 8 x 2^-25 at worst: 1.5e-7."""
+    n = 200
+    op = _op(n, 60, 290, start=start, fov=90.0, method="raycasting", step_size=step)
+    assert _off(op.forward, np.ones((n, n), np.float32)) <= 1e-7
+    y, x = np.mgrid[0:n, 0:n] / n - 0.5
+    img = sum(m * ((x - a) ** 2 + (y + a) ** 2 < r) for m, a, r in ((0.02, 0.0, 0.15), (0.013, 0.1, 0.02), (0.03, -0.2, 0.01)))
+    assert _off(op.forward, img.astype(np.float32)) <= 1.5e-7
