@@ -119,6 +119,8 @@ PROTOTYPES = {
     "ctr_bp_plan_run_grad": [c_void_p, _P, _P, c_int, _P],
     "ctr_bp_plan_destroy": [c_void_p],
     "ctr_fp_par_2d_cast_prep": [_S(ParParam), c_double, _P, _P, _P, _P],
+    "ctr_fp_par_2d_cast_scratch": [_S(ParParam), c_double],
+    "ctr_fp_par_2d_cast_f32_scratch": [_S(ParParam), c_double, _P, _P, _P, _P, _P, c_int, _P, ctypes.c_size_t, _P],
     "ctr_fp_par_2d_dd_prep": [_S(ParParam), _P, _P, _P, _P],
     "ctr_fp_par_2d_dd_grad_prep": [_S(ParParam), _P, _P, _P, _P],
     "ctr_ramp_filter_tc_create": [_S(FilterParam), _P, _S(FanWeightingParam), c_int, c_int, c_int,
@@ -155,7 +157,8 @@ for _t in ("f32", "f64"):
         f"ctr_helical_interpolation_180_{_t}": [_S(HelicalParam), _P, _P, _P, _P, c_int, _P],
     })
 _RESTYPES = {"ctr_status_string": c_char_p, "ctr_last_error": c_char_p,
-             "ctr_helical_interpolation_table_bytes": ctypes.c_size_t}
+             "ctr_helical_interpolation_table_bytes": ctypes.c_size_t,
+             "ctr_fp_par_2d_cast_scratch": ctypes.c_size_t}
 
 _lock = threading.Lock()
 _lib = None

@@ -320,46 +320,75 @@ int check_cast(const ctr_par_param* p, double step_size, const void* a, const vo
 // Steps up to this many pixels go row by row (fp_cast_rows_f32): the time does
 // not depend on the step there, that of the sample-by-sample kernel does.  Per
 // call (copies included), row by row against sample by sample:
-//   512^2 x 720 x 729   step 0.125: 393 / 2450 us, 0.5: 393 / 1176, 0.75: 393 / 1040
-//   128^2 x 180 x 190   step 0.125: 51 / 135 us,   0.5: 41 / 57,    0.75: 40 / 45
-//   64^2 x 90 x 96      step 0.125: 34 / 70 us,    0.5: 30 / 33,    0.75: 31 / 28
+//   512^2 x 720 x 729   step 0.125: 403 / 2450 us, 0.5: 403 / 1176
+//   128^2 x 180 x 190   step 0.125: 51 / 135 us,   0.5: 41 / 57
+//   64^2 x 90 x 96      step 0.125: 34 / 70 us,    0.5: 30 / 33
+// (At 0.75 the larger two would gain too, 403 / 1040 and 40 / 45, the last would
+// not, 31 / 28: those steps are left sample by sample.)
 // Geometries of fewer samples than kCastRowSamples (rays times the image's shorter
 // side in steps; an item's path is the same in any batch) are launches, of which the
 // copies are one more: 32^2 x 30 x 45 at a step of 0.25 23 / 19 us, 16^2 x 12 x 21
-// 21 / 15.
-constexpr double kCastRowStep = 0.5, kCastRowSamples = 5e5;
-constexpr int kCastNotRows = -1;
+// 21 / 15.  Where the call allocates the copies itself, a synchronisation between
+// calls has the pool give the memory back, and the next call takes ~170 us to get
+// it: kCastOwnSamples (341^2 x 457 x 424 at 0.125, 5e8: 344 / 900 us with such a
+// synchronisation; 183^2 x 255 x 267 at 0.5, 2.5e7: 256 / 95).
+constexpr double kCastRowStep = 0.5, kCastRowSamples = 5e5, kCastOwnSamples = 2e8;
+constexpr size_t kCastOwnBytes = 256u << 20;  // copies at a time of a call that allocates them
 
-// The row-by-row path of an FP32 call, kCastNotRows where it does not take it.
-int cast_rows(const ctr_par_param* p, double step_size, const float* img, float* proj, const double* sc,
-              const double* begins, const int* nsteps, float scale, int batch, cudaStream_t stream)
+// Bytes of an image's two copies; 0 where an FP32 call goes sample by sample.
+size_t cast_copies(const ctr_par_param* p, double step_size, double samples)
 {
     const size_t wx = static_cast<size_t>(p->nx) + 2 * kCastPad, wy = static_cast<size_t>(p->ny) + 2 * kCastPad;
-    const unsigned chunks = div_up(p->ns, kRowThreads);
-    const size_t blocks = static_cast<size_t>(chunks) * p->na;
     // the march indexes a copy with 32-bit integers
-    if (step_size > kCastRowStep || wx * wy > 0x7fffffffu || blocks > 0x7fffffffu) return kCastNotRows;
-    if (static_cast<double>(p->na) * p->ns * std::min(p->nx, p->ny) < kCastRowSamples * step_size) return kCastNotRows;
-    float* rows = nullptr;
-    const size_t item = wx * wy;
-    if (cudaMallocAsync(reinterpret_cast<void**>(&rows), 2 * sizeof(float) * item * batch, stream) != cudaSuccess) {
-        cudaGetLastError();  // no room for the copies: sample by sample
-        return kCastNotRows;
+    if (step_size > kCastRowStep || wx * wy > 0x7fffffffu ||
+        static_cast<size_t>(div_up(p->ns, kRowThreads)) * p->na > 0x7fffffffu)
+        return 0;
+    if (static_cast<double>(p->na) * p->ns * std::min(p->nx, p->ny) < samples * step_size) return 0;
+    return 2 * sizeof(float) * wx * wy;
+}
+
+// An FP32 call row by row, `most` images at a time with their copies in `scratch`.
+int cast_rows(const ctr_par_param* p, double step_size, const float* img, float* proj, const double* sc,
+              const double* begins, const int* nsteps, int batch, float* scratch, int most, cudaStream_t stream)
+{
+    const int nx = static_cast<int>(p->nx), ny = static_cast<int>(p->ny);
+    const unsigned wx = p->nx + 2 * kCastPad, wy = p->ny + 2 * kCastPad, chunks = div_up(p->ns, kRowThreads);
+    const size_t is = static_cast<size_t>(nx) * ny, ps = static_cast<size_t>(p->na) * p->ns;
+    for (int i = 0; i < batch; i += most) {
+        const unsigned count = std::min(most, batch - i);
+        float* cols = scratch + static_cast<size_t>(wx) * wy * count;
+        cast_pad<<<dim3(div_up(wx, 32), std::min(div_up(wy, 32), 32768u), count), 256, 0, stream>>>(img + i * is, scratch,
+                                                                                                    cols, nx, ny);
+        fp_cast_rows_f32<<<dim3(chunks * p->na, count), kRowThreads, 0, stream>>>(
+            scratch, cols, proj + i * ps, sc, begins, nsteps, p->ns, nx, ny, chunks, step_size,
+            static_cast<float>(step_size * p->dx), ps);
     }
-    float* cols = rows + item * batch;
-    cast_pad<<<dim3(div_up(wx, 32), std::min<size_t>(div_up(wy, 32), 32768), batch), 256, 0, stream>>>(
-        img, rows, cols, static_cast<int>(p->nx), static_cast<int>(p->ny));
-    fp_cast_rows_f32<<<dim3(static_cast<unsigned>(blocks), batch), kRowThreads, 0, stream>>>(
-        rows, cols, proj, sc, begins, nsteps, p->ns, p->nx, p->ny, chunks, step_size, scale,
-        static_cast<size_t>(p->na) * p->ns);
-    const int st = check_launch("fp_par_2d ray casting");
-    cudaFreeAsync(rows, stream);  // after the kernel that reads it
-    return st;
+    return check_launch("fp_par_2d ray casting");
+}
+
+// The row-by-row path with copies of the call's own; false where there is none, or
+// no room for one image's.
+bool cast_own_rows(const ctr_par_param* p, double step_size, const float* img, float* proj, const double* sc,
+                   const double* begins, const int* nsteps, int batch, cudaStream_t stream, int* status)
+{
+    const size_t item = cast_copies(p, step_size, kCastOwnSamples);
+    if (item == 0) return false;
+    int most = static_cast<int>(std::max<size_t>(1, std::min<size_t>(batch, kCastOwnBytes / item)));
+    float* scratch = nullptr;
+    while (cudaMallocAsync(reinterpret_cast<void**>(&scratch), item * most, stream) != cudaSuccess) {
+        cudaGetLastError();
+        if (most == 1) return false;
+        most = (most + 1) / 2;
+    }
+    *status = cast_rows(p, step_size, img, proj, sc, begins, nsteps, batch, scratch, most, stream);
+    cudaFreeAsync(scratch, stream);  // after the kernel that reads it
+    return true;
 }
 
 template <typename T>
 int cast_forward(const ctr_par_param* p, double step_size, const T* img, T* proj, const double* sc,
-                 const double* begins, const int* nsteps, int batch, cudaStream_t stream)
+                 const double* begins, const int* nsteps, int batch, cudaStream_t stream, bool own = true,
+                 void* scratch = nullptr, size_t bytes = 0)
 {
     int st = check_cast(p, step_size, img, proj, sc, begins, nsteps, batch);
     if (st) return st;
@@ -367,11 +396,13 @@ int cast_forward(const ctr_par_param* p, double step_size, const T* img, T* proj
     const dim3 grid(static_cast<unsigned>(div_up(static_cast<unsigned long long>(rays), kCastThreads)), batch);
     const size_t is = static_cast<size_t>(p->nx) * p->ny, ps = static_cast<size_t>(p->na) * p->ns;
     if constexpr (sizeof(T) == 4) {
-        const float scale = static_cast<float>(step_size * p->dx);
-        const int rc = cast_rows(p, step_size, img, proj, sc, begins, nsteps, scale, batch, stream);
-        if (rc != kCastNotRows) return rc;
-        fp_cast_f32<<<grid, kCastThreads, 0, stream>>>(img, proj, sc, begins, nsteps, p->ns, p->na, p->nx, p->ny,
-                                                       step_size, scale, is, ps);
+        if (own && cast_own_rows(p, step_size, img, proj, sc, begins, nsteps, batch, stream, &st)) return st;
+        const size_t item = cast_copies(p, step_size, kCastRowSamples);
+        if (item > 0 && bytes >= item)
+            return cast_rows(p, step_size, img, proj, sc, begins, nsteps, batch, static_cast<float*>(scratch),
+                             static_cast<int>(std::min<size_t>(batch, bytes / item)), stream);
+        fp_cast_f32<<<grid, kCastThreads, 0, stream>>>(img, proj, sc, begins, nsteps, p->ns, p->na, p->nx, p->ny, step_size,
+                                                       static_cast<float>(step_size * p->dx), is, ps);
     } else
         fp_cast_f64<<<grid, kCastThreads, 0, stream>>>(img, proj, sc, begins, nsteps, p->ns, p->na, p->nx, p->ny,
                                                        step_size, p->dx, is, ps);
@@ -446,6 +477,20 @@ int ctr_fp_par_2d_cast_f32(const ctr_par_param* p, double step_size, const float
                            cudaStream_t stream)
 {
     return cast_forward<float>(p, step_size, img, proj, sincostbl, begins, nsteps, batch, stream);
+}
+
+size_t ctr_fp_par_2d_cast_scratch(const ctr_par_param* p, double step_size)
+{
+    return p && p->nx > 0 && p->ny > 0 && step_size > 0.0 ? cast_copies(p, step_size, kCastRowSamples) : 0;
+}
+
+int ctr_fp_par_2d_cast_f32_scratch(const ctr_par_param* p, double step_size, const float* img, float* proj,
+                                   const double* sincostbl, const double* begins, const int* nsteps, int batch,
+                                   void* scratch, size_t bytes, cudaStream_t stream)
+{
+    if (bytes > 0 && (bad_ptr(scratch) || reinterpret_cast<uintptr_t>(scratch) % sizeof(float) != 0))
+        return fail(CTR_ERR_INVALID_ARG, "scratch null or not aligned to a float");
+    return cast_forward<float>(p, step_size, img, proj, sincostbl, begins, nsteps, batch, stream, false, scratch, bytes);
 }
 
 int ctr_fp_par_2d_cast_f64(const ctr_par_param* p, double step_size, const double* img, double* proj,

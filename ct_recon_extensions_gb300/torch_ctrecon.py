@@ -28,6 +28,7 @@ from ._lib import (FanBpAngleParam, FanBpParam, FanWeightingParam, FilterParam, 
 
 _FILTER_TYPES = {"par": 0, "fan": 1, "flat": 2}
 _WEIGHT_TYPES = {"fan": 1, "flat": 2}
+_CAST_BYTES = 256 << 20  # a ray-casting call's image copies at a time
 
 
 def _stream() -> int:
@@ -522,10 +523,30 @@ class ParallelProjection2DOp:
             return w, pos, ux
         return self._adj_tables.get(device, build)
 
+    def _cast_scratch(self, xb):
+        """Memory for the copies of the images that an FP32 ray-casting call
+        reads, of at most _CAST_BYTES or one image's at a time; None where it
+        needs none, or there is no room (the call then goes sample by sample).
+        From torch's allocator, which keeps it at a synchronisation."""
+        one = self._lib.ctr_fp_par_2d_cast_scratch(ctypes.byref(self.p), self.step_size)
+        count = min(xb.shape[0], max(1, _CAST_BYTES // one)) if one else 0
+        while count:
+            try:
+                return torch.empty(count * one, dtype=torch.uint8, device=xb.device)
+            except torch.cuda.OutOfMemoryError:
+                count //= 2
+        return None
+
     def forward(self, img):
         xb, restore = _as_batch(img, self.ny, self.nx, "fp_par_2d")
         proj = torch.empty((xb.shape[0], self.na, self.ns), dtype=xb.dtype, device=xb.device)
-        if self.method == "raycasting":
+        if self.method == "raycasting" and xb.dtype == torch.float32:
+            tables = self.tables(xb.device)
+            scratch = self._cast_scratch(xb)
+            call("ctr_fp_par_2d_cast_f32_scratch", ctypes.byref(self.p), self.step_size, _ptr(xb),
+                 _ptr(proj), *map(_ptr, tables), xb.shape[0], 0 if scratch is None else _ptr(scratch),
+                 0 if scratch is None else scratch.numel(), _stream())
+        elif self.method == "raycasting":
             call(f"ctr_fp_par_2d_cast_{_sfx(xb)}", ctypes.byref(self.p), self.step_size, _ptr(xb),
                  _ptr(proj), *map(_ptr, self.tables(xb.device)), xb.shape[0], _stream())
         elif self.method == "disdriven":

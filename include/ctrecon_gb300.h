@@ -315,12 +315,22 @@ int ctr_fp_par_2d_plan_destroy(ctr_fp_plan* plan);
  * sincostbl double[na][2], begins double[na][ns][2] (the ray's entry point on
  * the FoV circle of radius fov, in pixel indices), nsteps int[na][ns].
  * Forward (ParallelProjection2DRayCasting): samples every step_size pixels;
- * the reference has no gradient for this method. */
+ * the reference has no gradient for this method.  FP32 calls at steps up to
+ * half a pixel read copies of the images: ctr_fp_par_2d_cast_f32 takes their
+ * memory from the device's default pool where that pays, and otherwise does
+ * without; ctr_fp_par_2d_cast_f32_scratch uses the caller's, as many images at
+ * a time as `bytes` holds (ctr_fp_par_2d_cast_scratch bytes each; 0 where they
+ * are not used), and allocates nothing. */
 int ctr_fp_par_2d_cast_prep(const ctr_par_param* p, double step_size, double* sincostbl,
                             double* begins, int* nsteps, cudaStream_t stream);
 int ctr_fp_par_2d_cast_f32(const ctr_par_param* p, double step_size, const float* img,
                            float* proj, const double* sincostbl, const double* begins,
                            const int* nsteps, int batch, cudaStream_t stream);
+size_t ctr_fp_par_2d_cast_scratch(const ctr_par_param* p, double step_size);
+int ctr_fp_par_2d_cast_f32_scratch(const ctr_par_param* p, double step_size, const float* img,
+                                   float* proj, const double* sincostbl, const double* begins,
+                                   const int* nsteps, int batch, void* scratch, size_t bytes,
+                                   cudaStream_t stream);
 int ctr_fp_par_2d_cast_f64(const ctr_par_param* p, double step_size, const double* img,
                            double* proj, const double* sincostbl, const double* begins,
                            const int* nsteps, int batch, cudaStream_t stream);
