@@ -110,19 +110,20 @@ __device__ T dd_ray_exact(const T* __restrict__ I, const double* __restrict__ b,
     return sum;
 }
 
-// FP64 forward: the reference's loop, one thread per ray.
+// The reference's loop, one thread per ray: FP64, and FP32 where there is no room
+// for an image's copies.
+template <typename T>
 __global__ void __launch_bounds__(kDdThreads)
-    fp_dd_f64(const double* __restrict__ img, double* __restrict__ proj, const double* __restrict__ sincos,
-              const double* __restrict__ bo, const int* __restrict__ usex, int ns, int na, int nx, int ny,
-              double dx, double dy, size_t img_stride, size_t proj_stride)
+    fp_dd_rays(const T* __restrict__ img, T* __restrict__ proj, const double* __restrict__ sincos,
+               const double* __restrict__ bo, const int* __restrict__ usex, int ns, int na, int nx, int ny,
+               double dx, double dy, size_t img_stride, size_t proj_stride)
 {
     const long long ray = static_cast<long long>(blockIdx.x) * kDdThreads + threadIdx.x;
     if (ray >= static_cast<long long>(na) * ns) return;
     const int ia = static_cast<int>(ray / ns);
     const int ux = usex[ia];
-    const double w = ux ? fabs(dy / sincos[2 * ia + 1]) : fabs(dx / sincos[2 * ia]);
-    const double sum = dd_ray_exact<double>(img + blockIdx.y * img_stride, bo + 3 * ray, ux, ux ? ny : nx,
-                                            ux ? nx : ny, nx);
+    const T w = static_cast<T>(ux ? fabs(dy / sincos[2 * ia + 1]) : fabs(dx / sincos[2 * ia]));
+    const T sum = dd_ray_exact<T>(img + blockIdx.y * img_stride, bo + 3 * ray, ux, ux ? ny : nx, ux ? nx : ny, nx);
     proj[blockIdx.y * proj_stride + ray] = sum * w;
 }
 
@@ -876,13 +877,15 @@ int dd_forward(const ctr_par_param* p, const T* img, T* proj, const double* sc, 
     const unsigned long long rays = static_cast<unsigned long long>(p->na) * p->ns;
     const size_t is = static_cast<size_t>(p->nx) * p->ny, ps = static_cast<size_t>(p->na) * p->ns;
     const dim3 grid(div_up(rays, kDdThreads), batch);
-    if constexpr (sizeof(T) == 8) {
-        fp_dd_f64<<<grid, kDdThreads, 0, stream>>>(img, proj, sc, bo, usex, p->ns, p->na, p->nx, p->ny, p->dx,
-                                                   p->dy, is, ps);
+    auto by_rays = [&] {
+        fp_dd_rays<T><<<grid, kDdThreads, 0, stream>>>(img, proj, sc, bo, usex, p->ns, p->na, p->nx, p->ny, p->dx, p->dy,
+                                                       is, ps);
         return check_launch("fp_par_2d distance driven");
+    };
+    if constexpr (sizeof(T) == 8) {
+        return by_rays();
     } else {
         const int n = static_cast<int>(p->nx);
-        if (batch > 65535) return fail(CTR_ERR_UNSUPPORTED, "batch > 65535");
         float* rows = nullptr;
         const size_t copy = static_cast<size_t>(n) * (n + kDdPad);
         int most = batch;  // images at a time: fewer where there is no room for every one's copies
@@ -891,6 +894,10 @@ int dd_forward(const ctr_par_param* p, const T* img, T* proj, const double* sc, 
             cudaGetLastError();
             most = (most + 1) / 2;
             e = cudaMallocAsync(reinterpret_cast<void**>(&rows), 2 * sizeof(float) * copy * most, stream);
+        }
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            return by_rays();
         }
         if (e != cudaSuccess) return fail(CTR_ERR_CUDA, "distance-driven scratch: %s", cudaGetErrorString(e));
         const unsigned tiles = div_up(n + kDdPad, 32), chunks = div_up(p->ns, kDdRayThreads);
