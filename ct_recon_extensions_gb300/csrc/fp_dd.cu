@@ -943,25 +943,41 @@ int dd_grad_by_tiles(const ctr_par_param* p, const float* proj, float* img, cons
             len = l;
         }
     }
-    if (tiles_y > 65535 || static_cast<long long>(segs) * batch > 65535) return kDgNotTiles;
-    const size_t image = static_cast<size_t>(n) * n, count = image * batch;
-    const size_t part_at = (sizeof(DdView) * na + 255) / 256 * 256;
+    if (tiles_y > 65535) return kDgNotTiles;
+    // Images at a time: as many as the grid takes, fewer where there is no room for
+    // their partial images (an image's sums stay the same), and without partial
+    // images where there is none for one's.
+    const size_t image = static_cast<size_t>(n) * n, part_at = (sizeof(DdView) * na + 255) / 256 * 256;
+    int most = std::min(batch, 65535 / segs);
     char* scratch = nullptr;
-    if (cudaMallocAsync(reinterpret_cast<void**>(&scratch), part_at + (segs > 1 ? sizeof(float) * segs * count : 0),
-                        stream) != cudaSuccess) {
-        cudaGetLastError();  // no room for the partial images
-        return kDgNotTiles;
+    while (cudaMallocAsync(reinterpret_cast<void**>(&scratch),
+                           part_at + (segs > 1 ? sizeof(float) * segs * image * most : 0), stream) != cudaSuccess) {
+        cudaGetLastError();
+        if (segs == 1) return kDgNotTiles;
+        if (most > 1) {
+            most = (most + 1) / 2;
+        } else {
+            segs = 1;
+            len = blocks;
+            most = batch;
+        }
     }
     DdView* views = reinterpret_cast<DdView*>(scratch);
-    float* part = segs > 1 ? reinterpret_cast<float*>(scratch + part_at) : img;
     dd_grad_views<<<div_up(na, 8), 256, 0, stream>>>(pos, w, usex, views, na, n);
-    dd_grad_tiles<<<dim3(tiles_x, tiles_y, segs * batch), kDgThreads, 0, stream>>>(
-        proj, part, pos, views, static_cast<int>(p->ns), na, n, segs, len * kDgViews, count, image);
-    if (segs > 1)
-        dd_grad_sum<<<std::min<size_t>(div_up(count, 256), 8u * device_sms()), 256, 0, stream>>>(part, img, count, segs);
     const int groups = div_up(n, 32);
-    dd_grad_border<<<dim3(4 * groups, batch), kDbThreads, 0, stream>>>(proj, img, pos, views, static_cast<int>(p->ns),
-                                                                       na, n, groups);
+    for (int i = 0; i < batch; i += most) {
+        const int some = std::min(most, batch - i);
+        const size_t count = image * some;
+        const float* P = proj + static_cast<size_t>(i) * p->na * p->ns;
+        float* out = img + i * image;
+        float* part = segs > 1 ? reinterpret_cast<float*>(scratch + part_at) : out;
+        dd_grad_tiles<<<dim3(tiles_x, tiles_y, segs * some), kDgThreads, 0, stream>>>(
+            P, part, pos, views, static_cast<int>(p->ns), na, n, segs, len * kDgViews, count, image);
+        if (segs > 1)
+            dd_grad_sum<<<std::min<size_t>(div_up(count, 256), 8u * device_sms()), 256, 0, stream>>>(part, out, count, segs);
+        dd_grad_border<<<dim3(4 * groups, some), kDbThreads, 0, stream>>>(P, out, pos, views, static_cast<int>(p->ns), na, n,
+                                                                         groups);
+    }
     const int st = check_launch("fp_par_2d distance-driven grad");
     cudaFreeAsync(scratch, stream);  // after the kernels that read it
     return st;
