@@ -644,19 +644,24 @@ __global__ void __launch_bounds__(kSvThreads)
 // segment's middle pixel in FP64 from the caller's tables (integer part and
 // FP32 fraction), then steps through the segment in FP32 with the view's
 // slope, so every store of the warp writes 32 consecutive views of one pixel
-// (128 contiguous bytes).  The reference's inclusion rule 0 <= s <= ns-1 is
-// decided in FP64 (src/bp_par_2d_sv.cc:55-92 arithmetic) for positions within
-// a channel of a detector end; farther out the output is 0, farther in the
-// FP32 position (within ~4e-6 channels) interpolates.
+// (128 contiguous bytes).  The reference's inclusion rule 0 <= s <= ns-1
+// (src/bp_par_2d_sv.cc:55-92) is decided from the position in two floats within
+// a channel of a detector end, and in FP64, with the reference's operations,
+// within 1e-5 of it; farther out the output is 0, farther in the FP32 position
+// (within ~4e-6 channels) interpolates.  (FP64 throughout that channel, which some
+// lane of a warp is in at nearly every pixel of a row's ends, took most of the
+// time where the detector is shorter than the image's diagonal: 300^2 x 720 from
+// 301 channels 320 us, 475^2 x 720 from 572 373, now 98 and 251.)
 // Inside the detector a lane walks its channels in the direction they change
 // along the segment, less than two a pixel, and keeps the two it is between: it
 // loads one when it passes a channel, where two loads a pixel made the shared
-// loads the bound.  The rows are dealt evenly over as many CTAs as fill the
-// resident ones (16 rows a CTA were 2.4 waves of them).  720 x 729 -> 512^2 x
-// 720: 188 -> 153 us (filling the output takes 99 us); issue bound now (61 %).
+// loads the bound.  A row's segments are of equal length, so that the warps are
+// even.  720 x 729 -> 512^2 x 720: 188 -> 158 us (filling the output takes 99 us);
+// issue bound now.
 constexpr int kSvFastThreads = 512;
 constexpr int kSvViews = 32;
 constexpr int kSvSeg = 64;
+constexpr double kSvL2Bytes = 100e6;  // output that stays in L2 (129 MB)
 
 // One step of the walk: the channel numbered `b` lies at or past the last one's
 // `bp`; near and far become the values before and after the position (far at
@@ -692,6 +697,7 @@ __global__ void __launch_bounds__(kSvFastThreads, 2)
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane >= nv) return;  // no barrier follows
+    const unsigned lanes = nv == 32 ? 0xffffffffu : (1u << nv) - 1;
     const int ia = v0 + lane;
     const float* R = sv_rows + lane * stride;
     // the view's channel step per pixel along x, from the caller's x cos t table
@@ -705,7 +711,8 @@ __global__ void __launch_bounds__(kSvFastThreads, 2)
     const int segs = (nx + kSvSeg - 1) / kSvSeg;
     for (int task = warp; task < (y1 - y0) * segs; task += kSvFastThreads / 32) {
         const int iy = y0 + task / segs;
-        const int xs0 = (task % segs) * kSvSeg, xs1 = min(nx, xs0 + kSvSeg);
+        const int seg = task % segs;
+        const int xs0 = nx * seg / segs, xs1 = nx * (seg + 1) / segs;
         const int xm = (xs0 + xs1) / 2;
         const double ys = ysin[static_cast<size_t>(iy) * na + ia];
         const double sd0 = (xcos[static_cast<size_t>(xm) * na + ia] + ys) * inv_ds + cents;
@@ -715,11 +722,11 @@ __global__ void __launch_bounds__(kSvFastThreads, 2)
         const float fh = static_cast<float>(sd0 - fl0) - 0.5f;
         float* Or = O + (static_cast<size_t>(iy) * nx + xs0) * ostep;
         // the position is linear along the segment: interior when both ends are
-        // at least a channel inside the detector
+        // at least a channel inside the detector, for every lane's view
         const float ka = static_cast<float>(xs0 - xm), kb = static_cast<float>(xs1 - 1 - xm);
         const int ja = i0 + static_cast<int>(floorf(fmaf(ka, px, fh) + 0.5f));
         const int jb = i0 + static_cast<int>(floorf(fmaf(kb, px, fh) + 0.5f));
-        if (min(ja, jb) >= 1 && max(ja, jb) <= ns - 3) {
+        if (__all_sync(lanes, min(ja, jb) >= 1 && max(ja, jb) <= ns - 3)) {
             // t: the way along dir past the reference (i0 + 1/2), r its integer
             const float t0 = px < 0.0f ? -fh : fh, ap = fabsf(px);
             // the address of the channel after the one numbered by the bits of r + kMagic
@@ -752,6 +759,11 @@ __global__ void __launch_bounds__(kSvFastThreads, 2)
             }
             continue;
         }
+        // the reference's place past i0 and the step in two floats (the step from this
+        // segment's pixels: formed here, it takes no registers from the walk)
+        const float f0 = static_cast<float>(sd0 - fl0), f0_low = static_cast<float>((sd0 - fl0) - f0);
+        const size_t x1 = static_cast<size_t>(xs0) * na + ia, x2 = static_cast<size_t>(xs1 - 1) * na + ia;
+        const float px_low = static_cast<float>((xcos[x2] - xcos[x1]) * inv_ds / max(1, xs1 - 1 - xs0) - px);
         float kf = ka;
         for (int ix = xs0; ix < xs1; ++ix, kf += 1.0f, Or += ostep) {
             const float sr = fmaf(kf, px, fh);
@@ -761,19 +773,36 @@ __global__ void __launch_bounds__(kSvFastThreads, 2)
             float out = 0.0f;
             bool in = j >= 1 && j <= ns - 3;
             if (!in && j >= -1 && j <= ns) {
-                // within a channel of an end: the reference's FP64 decision
-                const double sd = (xcos[static_cast<size_t>(ix) * na + ia] + ys) / ds + cents;
-                in = sd >= 0.0 && sd <= static_cast<double>(ns - 1);
-                if (in) {
-                    const double f = floor(sd);
-                    j = static_cast<int>(f);
-                    u = static_cast<float>(sd - f);
+                // f0 + kf step in two floats
+                const float h = kf * px, r = f0 + h, b = r - f0;
+                const float low = ((f0 - (r - b)) + (h - b)) + (fmaf(kf, px, -h) + fmaf(kf, px_low, f0_low));
+                const float fl = floorf(r);
+                j = i0 + static_cast<int>(fl);
+                u = (r - fl) + low;
+                if (u < 0.0f) {
+                    --j;
+                    u += 1.0f;
+                } else if (u >= 1.0f) {
+                    ++j;
+                    u -= 1.0f;
+                }
+                in = j >= 0 && j <= ns - 2;
+                const int at_end = u < 0.5f ? j : j + 1;
+                if ((at_end == 0 || at_end == ns - 1) && fabsf(u - static_cast<float>(at_end - j)) < 1e-5f) {
+                    const double sd = (xcos[static_cast<size_t>(ix) * na + ia] + ys) / ds + cents;
+                    in = sd >= 0.0 && sd <= static_cast<double>(ns - 1);
+                    if (in) {
+                        const double f = floor(sd);
+                        j = static_cast<int>(f);
+                        u = static_cast<float>(sd - f);
+                    }
                 }
             }
             if (in) {
                 const float a = R[j], b = R[min(j + 1, ns - 1)];
                 out = fmaf(u, b - a, a);
             }
+            __syncwarp(lanes);  // one store of the warp
             *Or = out;
         }
     }
@@ -1198,19 +1227,32 @@ int par_single_view(const ctr_par_param* p, const T* proj, T* img, const double*
             cudaError_t e = cudaFuncSetAttribute(bp_par_sv_f32, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  static_cast<int>(smem));
             if (e != cudaSuccess) return fail(CTR_ERR_CUDA, "bp_par_2d_sv: %s", cudaGetErrorString(e));
-            // Bands of rows for the fewest rows on the busiest CTA slot (a CTA's
-            // staging costs about a row).
-            const long long tiles = static_cast<long long>(div_up(p->na, kSvViews)) * batch;
-            const int slots = (smem <= kTileSmemMax ? 2 : 1) * sm_count(), ny = static_cast<int>(p->ny);
+            // Bands of rows.  Where every store fills whole sectors (32 bytes: na a
+            // multiple of 8), or the output stays in L2, the fewest rounds of a CTA's warps
+            // on the busiest CTA slot, its staging half a round (512^2 x 720 above: 179 us
+            // with 16 rows a CTA).  Else neighbouring view tiles share sectors, which have
+            // to meet in L2 before they are written back: two segments a warp, so that the
+            // tiles stay together (512^2 x 721: 265 us, 329 in the fewest bands, 324 with
+            // 16 rows; 160^2 x 709, 73 MB: 34 so, 29, 32), three for narrow images where
+            // half of the sectors are one tile's own (3 x 160^2 x 700: 69 us with two, 66).
+            const int segs = div_up(p->nx, kSvSeg), ny = static_cast<int>(p->ny), warps = kSvFastThreads / 32;
             int bands = 1;
-            double best = 1e300;
-            for (int b = 1; b <= std::min(ny, 64); ++b) {
-                const double cost = static_cast<double>((tiles * b + slots - 1) / slots) * ((ny + b - 1) / b + 1.0);
-                if (cost < best) {
-                    best = cost;
-                    bands = b;
+            if (p->na % 8 != 0 && sizeof(T) * p->nx * p->ny * static_cast<double>(p->na) * batch > kSvL2Bytes) {
+                bands = div_up(ny, std::max(1, (p->na % 4 == 0 && segs <= 3 ? 3 : 2) * warps / segs));
+            } else {
+                const long long tiles = static_cast<long long>(div_up(p->na, kSvViews)) * batch;
+                const int slots = (smem <= kTileSmemMax ? 2 : 1) * sm_count();
+                double best = 1e300;
+                for (int b = 1; b <= std::min(ny, 64); ++b) {
+                    const double cost = static_cast<double>((tiles * b + slots - 1) / slots) *
+                                        (div_up(static_cast<unsigned long long>(div_up(ny, b)) * segs, warps) + 0.5);
+                    if (cost < best) {
+                        best = cost;
+                        bands = b;
+                    }
                 }
             }
+            bands = std::min(bands, 65535);
             dim3 g2(div_up(p->na, kSvViews), bands, batch);
             bp_par_sv_f32<<<g2, kSvFastThreads, smem, stream>>>(
                 proj, img, xcos, ysin, p->ns, p->na, p->nx, p->ny, p->ds, 1.0 / p->ds, cents, stride,
