@@ -29,6 +29,7 @@
 #include <type_traits>
 
 #include "bp_tile.cuh"
+#include "sv_walk.h"
 
 namespace ctr {
 namespace {
@@ -661,6 +662,7 @@ __global__ void __launch_bounds__(kSvThreads)
 constexpr int kSvFastThreads = 512;
 constexpr int kSvViews = 32;
 constexpr int kSvSeg = 64;
+static_assert(kSvMagicBits == kMagicBits, "positions are rounded by kMagic");
 constexpr double kSvL2Bytes = 100e6;  // output that stays in L2 (129 MB)
 
 // One step of the walk: the channel numbered `b` lies at or past the last one's
@@ -730,15 +732,14 @@ __global__ void __launch_bounds__(kSvFastThreads, 2)
             // t: the way along dir past the reference (i0 + 1/2), r its integer
             const float t0 = px < 0.0f ? -fh : fh, ap = fabsf(px);
             // the address of the channel after the one numbered by the bits of r + kMagic
-            const unsigned at0 = at + 4u * static_cast<unsigned>(px < 0.0f ? i0 + 1 : i0) + static_cast<unsigned>(dir4) -
-                                 kMagicBits * static_cast<unsigned>(dir4);
+            const unsigned at0 = sv_base(at, px < 0.0f ? i0 + 1 : i0, dir4);
             const float2 t02 = make_float2(t0, t0), ap2 = make_float2(ap, ap), two2 = make_float2(2.0f, 2.0f);
             float2 kf = make_float2(ka, ka + 1.0f);
             int last = 0;  // no channel yet: any number lies more than one past it
             float near = 0.0f, far = 0.0f;
             auto value = [&](float vb, float u) {
                 const int num = __float_as_int(vb);
-                sv_advance(near, far, num, last, at0 + static_cast<unsigned>(num * dir4), dir4);
+                sv_advance(near, far, num, last, sv_address(at0, num, dir4), dir4);
                 last = num;
                 return fmaf(u, far - near, near);
             };
