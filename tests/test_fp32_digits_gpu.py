@@ -96,3 +96,28 @@ def test_ray_casting(step, start):
     y, x = np.mgrid[0:n, 0:n] / n - 0.5
     img = sum(m * ((x - a) ** 2 + (y + a) ** 2 < r) for m, a, r in ((0.02, 0.0, 0.15), (0.013, 0.1, 0.02), (0.03, -0.2, 0.01)))
     assert _off(op.forward, img.astype(np.float32)) <= 1.5e-7
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 3.3e38])
+@pytest.mark.parametrize("method", ["360", "180"])
+def test_helical_not_finite(method, value):
+    """Infinities and NaN in a scan reach the samples that they reach in FP64, as
+    infinities where only measured rows have them (means of rows, 360LI)."""
+    from ct_recon_extensions_gb300 import torch_ctrecon as tc
+    ns, nt, vpr, nz = 130, 16, 300, 24
+    cm = nt * 595.0 / 1085.6 / vpr
+    op = tc.HelicalInterpolationOp(ns, nt, 4 * vpr, 900.0 / ns, 1.0, 0.375, -0.25, 0.0, 2 * math.pi / vpr, 0.0, cm, vpr, nz,
+                                   1.7 * vpr * cm / nz, (vpr + 3.3) * cm, 1.4, 595.0, 1085.6, method)
+    rng = np.random.default_rng(5)
+    x = rng.random((4 * vpr, nt, ns)).astype(np.float32)
+    x[rng.integers(vpr, 3 * vpr, 40), rng.integers(nt, size=40), rng.integers(ns, size=40)] = value
+    got, want = host(op.forward(cuda(x))), host(op.forward(cuda(x.astype(np.float64))))
+    if value == 3.3e38:
+        fine = np.abs(want) < 1e30
+        assert rel_l2(got[fine], want[fine]) <= 1e-6
+        return
+    assert np.array_equal(np.isfinite(got), np.isfinite(want)) and not np.isfinite(want).all()
+    fine = np.isfinite(want)
+    assert rel_l2(got[fine], want[fine]) <= 1e-6
+    if method == "360":
+        assert np.array_equal(np.isnan(got), np.isnan(want))
