@@ -575,8 +575,8 @@ __device__ __forceinline__ int ray_code(const FpxRays& r, const FpxConst& c, int
     return k0 | (k1 << 15);
 }
 
-// One image: 25.2e7 warp instructions of 15.8 a sample issue at 64 % of the
-// slots; the positions, fractions and addresses are half of them.  IMG = 2
+// One image: 84.3 M warp instructions, ~15 a sample and lane, issue at 62 % of
+// the slots; the positions, fractions and addresses are half of them.  IMG = 2
 // takes two images of a batch side by side, the second one's band kFpxSecond
 // floats behind the first's in a stage, and forms these once for both (16 x
 // 512^2, 720 views x 729: 1680 -> 1165 us).  Its bands are half as high; the

@@ -9,14 +9,15 @@
 // scaled by step_size * dx.
 //
 // FP32 path (fp_cast_rows_f32 for steps up to half a pixel, fp_cast_f32 above and
-// where the copies do not fit).  The sample range of each axis is decided exactly as the reference decides it: in 32.32 fixed point where that is
-// certain, and by the reference's own FP64 accumulation (acc_advance, jumping
-// binade to binade) for the few samples within a hair of an image edge
-// (fp_setup.cuh).  The running position is monotone in k, so each axis keeps a
-// contiguous range and the ray keeps their intersection.  Inside it both
-// coordinates are fixed point and the interpolation FP32; positions differ from the reference's FP64 ones by
-// ~1e-9 pixel, which moves the interpolation weights by as much (continuous at
-// pixel boundaries).
+// where an image's copies do not fit).  The sample range of each axis is decided
+// exactly as the reference decides it: in 32.32 fixed point where that is certain,
+// and by the reference's own FP64 accumulation (acc_advance, jumping binade to
+// binade) for the few samples within a hair of an image edge (fp_setup.cuh).  The
+// running position is monotone in k, so each axis keeps a contiguous range and the
+// ray keeps their intersection.  Inside it both coordinates are fixed point and the
+// interpolation FP32; positions differ from the reference's FP64 ones by ~1e-9
+// pixel, which moves the interpolation weights by as much (continuous at pixel
+// boundaries).
 //
 // FP64 path: one thread per ray, the reference's loop (FP64 positions and
 // inclusion test, FP64 interpolation and sum).
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(kCastThreads)
 // warp's pixels of a row are adjacent; rays marched in x read the transposed
 // copy.  Both copies have a border of kCastPad zeros around the image (the
 // fixed-point positions may sit a hair outside it, where the weight is ~0), so
-// the loop has no clamps.  Issue bound: ~75 instructions per ray and row, 67 %
+// the loop has no clamps.  Issue bound: ~75 instructions per ray and row, 66 %
 // of the issue slots (512^2 x 720 x 729 at a step of 0.125: 2450 -> 403 us).
 // Blocks start with the long rays of every view, near the detector's middle, and
 // end with short ones: view by view the SMs ran dry one by one (467 us).
