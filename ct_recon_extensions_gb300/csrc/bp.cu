@@ -1231,7 +1231,9 @@ int par_single_view(const ctr_par_param* p, const T* proj, T* img, const double*
             // Bands of rows.  Where every store fills whole sectors (32 bytes: na a
             // multiple of 8), or the output stays in L2, the fewest rounds of a CTA's warps
             // on the busiest CTA slot, its staging half a round (512^2 x 720 above: 179 us
-            // with 16 rows a CTA).  Else neighbouring view tiles share sectors, which have
+            // with 16 rows a CTA); of two about equal, the one of more waves, whose CTAs even
+            // out (768^2 x 360 from 1087 channels: 298 us in one wave, 226 in two, 273 with 16
+            // rows).  Else neighbouring view tiles share sectors, which have
             // to meet in L2 before they are written back: two segments a warp, so that the
             // tiles stay together (512^2 x 721: 265 us, 329 in the fewest bands, 324 with
             // 16 rows; 160^2 x 709, 73 MB: 34 so, 29, 32), three for narrow images where
@@ -1245,7 +1247,8 @@ int par_single_view(const ctr_par_param* p, const T* proj, T* img, const double*
                 const int slots = (smem <= kTileSmemMax ? 2 : 1) * sm_count();
                 double best = 1e300;
                 for (int b = 1; b <= std::min(ny, 64); ++b) {
-                    const double cost = static_cast<double>((tiles * b + slots - 1) / slots) *
+                    const double waves = static_cast<double>((tiles * b + slots - 1) / slots);
+                    const double cost = waves * (1.0 + 0.03 / waves) *
                                         (div_up(static_cast<unsigned long long>(div_up(ny, b)) * segs, warps) + 0.5);
                     if (cost < best) {
                         best = cost;
