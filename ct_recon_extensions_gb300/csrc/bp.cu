@@ -656,14 +656,14 @@ __global__ void __launch_bounds__(kSvThreads)
 // Inside the detector a lane walks its channels in the direction they change
 // along the segment, less than two a pixel, and keeps the two it is between: it
 // loads one when it passes a channel, where two loads a pixel made the shared
-// loads the bound.  A row's segments are of equal length, so that the warps are
-// even.  720 x 729 -> 512^2 x 720: 188 -> 158 us (filling the output takes 99 us);
+// loads the bound.  A row's segments are about equal, so that the warps are
+// even.  720 x 729 -> 512^2 x 720: 188 -> 155 us (filling the output takes 99 us);
 // issue bound now.
 constexpr int kSvFastThreads = 512;
 constexpr int kSvViews = 32;
 constexpr int kSvSeg = 64;
 static_assert(kSvMagicBits == kMagicBits, "positions are rounded by kMagic");
-constexpr double kSvL2Bytes = 100e6;  // output that stays in L2 (129 MB)
+constexpr double kSvL2Bytes = 130e6;  // about L2: output that stays there
 
 // One step of the walk: the channel numbered `b` lies at or past the last one's
 // `bp`; near and far become the values before and after the position (far at
@@ -710,11 +710,11 @@ __global__ void __launch_bounds__(kSvFastThreads, 2)
     const size_t ostep = static_cast<size_t>(na);
     const int y0 = static_cast<int>(static_cast<long long>(ny) * blockIdx.y / gridDim.y);
     const int y1 = static_cast<int>(static_cast<long long>(ny) * (blockIdx.y + 1) / gridDim.y);
-    const int segs = (nx + kSvSeg - 1) / kSvSeg;
+    // a row's segments: equal but for a multiple of four pixels
+    const int segs = (nx + kSvSeg - 1) / kSvSeg, len = ((nx + segs - 1) / segs + 3) & ~3;
     for (int task = warp; task < (y1 - y0) * segs; task += kSvFastThreads / 32) {
         const int iy = y0 + task / segs;
-        const int seg = task % segs;
-        const int xs0 = nx * seg / segs, xs1 = nx * (seg + 1) / segs;
+        const int xs0 = task % segs * len, xs1 = min(nx, xs0 + len);
         const int xm = (xs0 + xs1) / 2;
         const double ys = ysin[static_cast<size_t>(iy) * na + ia];
         const double sd0 = (xcos[static_cast<size_t>(xm) * na + ia] + ys) * inv_ds + cents;
@@ -1250,7 +1250,7 @@ int par_single_view(const ctr_par_param* p, const T* proj, T* img, const double*
                     const double waves = static_cast<double>((tiles * b + slots - 1) / slots);
                     const double cost = waves * (1.0 + 0.03 / waves) *
                                         (div_up(static_cast<unsigned long long>(div_up(ny, b)) * segs, warps) + 0.5);
-                    if (cost < best) {
+                    if (cost <= best) {  // shorter bands of as many rounds
                         best = cost;
                         bands = b;
                     }
