@@ -774,9 +774,10 @@ __global__ void __launch_bounds__(kSvFastThreads, 2)
             float out = 0.0f;
             bool in = j >= 1 && j <= ns - 3;
             if (!in && j >= -1 && j <= ns) {
-                // f0 + kf step in two floats
-                const float h = kf * px, r = f0 + h, b = r - f0;
-                const float low = ((f0 - (r - b)) + (h - b)) + (fmaf(kf, px, -h) + fmaf(kf, px_low, f0_low));
+                // f0 + kf step in two floats (no product fused into the sums)
+                const float h = __fmul_rn(kf, px), r = __fadd_rn(f0, h), b = __fadd_rn(r, -f0);
+                const float low = (__fadd_rn(f0, -__fadd_rn(r, -b)) + __fadd_rn(h, -b)) +
+                                  (fmaf(kf, px, -h) + fmaf(kf, px_low, f0_low));
                 const float fl = floorf(r);
                 j = i0 + static_cast<int>(fl);
                 u = (r - fl) + low;

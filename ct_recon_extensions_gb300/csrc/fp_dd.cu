@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kDdThreads)
 // block's lanes on adjacent channels of one view, the warp's rays on the same
 // line, so that each load reads adjacent pixels.  Blocks follow one another by
 // view, chunk of channels by chunk: neighbouring views' rays through the same
-// lines, and short rays at the detector's end for the last blocks (calls of 512^2 x
+// lines, and the short rays of the detector's first eighth for the last blocks (calls of 512^2 x
 // 720 x 729 with a quarter channel's offset: 284 us view by view, 260 so, three
 // images 703 and 667; without the offset 278 either way; from the middle outwards,
 // as in the ray casting, 320).  Issue bound.
